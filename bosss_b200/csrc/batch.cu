@@ -24,6 +24,7 @@
 #include "batch.h"
 #include "dg_slab_kernel.cuh"
 #include "handle.h"
+#include "modal.h"
 
 namespace bosss {
 
@@ -392,6 +393,7 @@ static int build_class_items(bosss_batch* b, int mode, int want) {
 
 static int batch_run(bosss_batch* b, int mode, double alpha, double beta, const double* U, const double* V, double* out,
                      double time, cudaStream_t s, int counter_slot) {
+    if (b->modal) return modal_batch_run(b->modal, mode, alpha, beta, U, V, out, s);
     if (b->classes) {
         for (const auto& r : b->runs[mode]) {
             ClassLaunch CL = class_launcher(b->phys, mode, r.K, r.Q, r.slab);
@@ -501,6 +503,13 @@ int bosss_b200_batch_create(int32_t n, const bosss_op_desc* ops, const bosss_gri
             return rc;
         }
     }
+    if (want == 0) {
+        const int rc = modal_batch_create(b->h, b->dom_off.data(), b->cod_off.data(), &b->modal);
+        if (rc) {
+            bosss_b200_batch_destroy(b);
+            return rc;
+        }
+    }
     *out = b;
     return BOSSS_OK;
 }
@@ -514,6 +523,7 @@ int bosss_b200_batch_destroy(bosss_batch* b) {
         cudaFree(b->d_items[m]);
         cudaFree(b->d_class_items[m]);
     }
+    modal_batch_destroy(b->modal);
     cudaFree(b->d_inst);
     cudaFree(b->d_counter);
     for (auto* h : b->h) bosss_b200_destroy(h);
@@ -671,6 +681,7 @@ int bosss_b200_batch_autotune(bosss_batch* b, const double* U_dev, const double*
         int best = 1;
         float best_ms = 1e30f;
         for (int r : {1, 2, 4, 8}) {
+            if (b->modal) break;   // one tile per CTA: nothing to time
             b->tiles[kq] = r;
             float ms = 0.f;
             rc = time_once(ms);
@@ -688,7 +699,7 @@ int bosss_b200_batch_autotune(bosss_batch* b, const double* U_dev, const double*
         if (have_sched) {
             b->lpt = lpt;
             b->classes = per_class;
-        } else {
+        } else if (!b->modal) {
             // persistent queue longest-first, persistent queue in instance order, or one launch
             // per (K, Q) class: the fastest of the three
             float ms_l = 0.f, ms_f = 0.f, ms_c = 0.f;

@@ -12,6 +12,7 @@
 namespace bosss {
 struct BatchInst;
 struct WorkItem;
+struct ModalBatch;
 }  // namespace bosss
 
 struct bosss_batch {
@@ -37,5 +38,6 @@ struct bosss_batch {
     bool classes = false;
     std::vector<ClassRun> runs[3];
     bosss::WorkItem* d_class_items[3] = {nullptr, nullptr, nullptr};
+    bosss::ModalBatch* modal = nullptr;           // linear instances: the modal kernel (no work queue)
     cudaGraphExec_t graph = nullptr;
 };

@@ -22,6 +22,7 @@
 #include "dg_registry.h"
 #include "bsr.h"
 #include "handle.h"
+#include "modal.h"
 #include "faces_euler.h"
 #include "tc_volume.h"
 
@@ -549,7 +550,10 @@ int bosss_b200_create(const bosss_op_desc* op, const bosss_grid_desc* grid, cons
     h->ncod = h->ndom;
     h->variant = VARIANT_GENERIC;   // generic unless some mode runs on the slab kernel
     for (int m = 0; m < 3; ++m) {
-        h->kern[m] = reg[KernelKey(phys, D, K, Q, m, mode_variant[m])];
+        // linear constant-coefficient scalar forms with an exact rule: the modal stencil kernel
+        if (want == 0 && prec == BOSSS_PRECISION_FP64 && modal_applies(phys, ph, K, Q)) mode_variant[m] = VARIANT_MODAL;
+        h->kern[m] = mode_variant[m] == VARIANT_MODAL ? modal_entry(phys, D, K, m)
+                                                      : reg[KernelKey(phys, D, K, Q, m, mode_variant[m])];
         h->kern_variant[m] = mode_variant[m];
         if (mode_variant[m] == VARIANT_SLAB) h->variant = VARIANT_SLAB;
     }
@@ -733,7 +737,7 @@ int bosss_b200_kernel_info(const bosss_handle* h, int32_t mode, int32_t* kernel,
     const bool split = mode == MODE_RES && h->precision == BOSSS_PRECISION_SPLIT_FP32;
     const bool once = h->faces_once && (mode == MODE_RES || mode == MODE_VJP);
     const bool slab = h->kern_variant[mode] == VARIANT_SLAB;
-    int k = slab ? 2 : 1, n = 1;
+    int k = slab ? 2 : (h->kern_variant[mode] == VARIANT_MODAL ? 5 : 1), n = 1;
     if (split) {
         k = 4;
         n = once ? 3 : 2;

@@ -1,0 +1,129 @@
+// modal.cu -- launches of the modal stencil kernel (modal_kernel.cuh) on one grid, and the tile
+// extents of a grid.
+#include <algorithm>
+
+#include "modal_kernel.cuh"
+
+namespace bosss {
+
+namespace {
+
+template <int D, int K, bool SIP, int MODE, bool MASK>
+__global__ void __launch_bounds__(MODAL_NT, ModalCfg<D, K>::MINB)
+k_modal(const __grid_constant__ EvalArgs a, const __grid_constant__ ModalTile tl) {
+    extern __shared__ double smem[];
+    modal_tile<D, K, SIP, MODE, MASK>(a, tl, blockIdx.x, MODE == MODE_RES ? a.U : a.V, a.out, a.alpha, a.beta, smem);
+}
+
+template <int D, int K, bool SIP, int MODE, bool MASK>
+cudaError_t launch_masked(const EvalArgs& a, cudaStream_t s) {
+    static unsigned long long done = 0ull;
+    const size_t smem = ModalCfg<D, K>::SMEM;
+    cudaError_t e = modal_attr(k_modal<D, K, SIP, MODE, MASK>, smem, done);
+    if (e != cudaSuccess) return e;
+    if (a.cend <= a.cbeg) return cudaSuccess;
+    const ModalTile tl = modal_tiling(a, D, K);
+    k_modal<D, K, SIP, MODE, MASK><<<tl.t[0] * tl.t[1] * tl.t[2], MODAL_NT, smem, s>>>(a, tl);
+    return cudaGetLastError();
+}
+
+template <int D, int K, bool SIP, int MODE>
+cudaError_t launch_modal(const EvalArgs& a, cudaStream_t s) {
+    // species masks (XDG) accompany the SIP residual only in practice; every mode reads them
+    if constexpr (SIP && D == 3)
+        if (a.vol_flag || a.face_flag) return launch_masked<D, K, SIP, MODE, true>(a, s);
+    return launch_masked<D, K, SIP, MODE, false>(a, s);
+}
+
+template <int D, int K, bool SIP>
+KernelEntry entry_of(int mode) {
+    KernelEntry e{nullptr, MODAL_NT, ModalCfg<D, K>::SMEM};
+    e.launch = mode == MODE_RES   ? &launch_modal<D, K, SIP, MODE_RES>
+               : mode == MODE_JVP ? &launch_modal<D, K, SIP, MODE_JVP>
+                                  : &launch_modal<D, K, SIP, MODE_VJP>;
+    return e;
+}
+
+template <int D>
+KernelEntry entry_dim(int phys, int K, int mode) {
+    if (phys == PHYS_TRANSPORT) switch (K) {
+            case 0: return entry_of<D, 0, false>(mode);
+            case 1: return entry_of<D, 1, false>(mode);
+            case 2: return entry_of<D, 2, false>(mode);
+            case 3: return entry_of<D, 3, false>(mode);
+            case 4: return entry_of<D, 4, false>(mode);
+        }
+    if (phys == PHYS_SIP) switch (K) {
+            case 1: return entry_of<D, 1, true>(mode);
+            case 2: return entry_of<D, 2, true>(mode);
+            case 3: return entry_of<D, 3, true>(mode);
+            case 4: return entry_of<D, 4, true>(mode);
+        }
+    return KernelEntry{nullptr, 0, 0};
+}
+
+}  // namespace
+
+KernelEntry modal_entry(int phys, int D, int K, int mode) {
+    return D == 2 ? entry_dim<2>(phys, K, mode) : entry_dim<3>(phys, K, mode);
+}
+
+ModalTile modal_tiling(const EvalArgs& a, int D, int K, bool shared) {
+    const GridConst& g = a.g;
+    const bool rev = D == 3 && g.stride[0] == 1 && g.stride[2] != 1;
+    const int n0 = rev ? g.n[2] : g.n[0], n1 = D == 3 ? g.n[1] : 1, n2 = D == 3 ? (rev ? g.n[0] : g.n[2]) : g.n[1];
+    const long long plane = (long long)n1 * n2;
+    const int s0 = (int)(a.cbeg / plane), s1 = (int)std::min<long long>(n0, (a.cend + plane - 1) / plane);
+    const int m0 = std::max(1, s1 - s0);
+    (void)K;
+    // the extents depend on the sizes alone: the last ones found on this thread are kept, since
+    // the search (a few hundred candidates) costs as much as a launch
+    struct Memo {
+        int D = 0, m0 = 0, n1 = 0, n2 = 0, shared = 0;
+        ModalTile t{};
+    };
+    static thread_local Memo memo;
+    if (memo.D == D && memo.m0 == m0 && memo.n1 == n1 && memo.n2 == n2 && memo.shared == (int)shared) {
+        ModalTile t = memo.t;
+        t.s0 = s0;
+        return t;
+    }
+    // extents within the halo box of the slots; the cost of a tile is its staged cells plus a fixed
+    // part (launch, latency), and CTAs run in waves of about 2 per SM
+    ModalTile best{};
+    double bc = 1e300;
+    const int c0[] = {1, 2, 3, 4, 5, 6, 8}, c2[] = {2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 16};
+    for (int b0 : c0)
+        for (int b1 : c0)
+            for (int b2 : c2) {
+                if (D == 2 && b1 != 1) continue;
+                if (b0 * b1 * b2 > MODAL_NT) continue;
+                if (D == 3 && (b0 + 2) * (b1 + 2) * (b2 + 2) > 6 * 6 * 10) continue;
+                if (D == 2 && (b0 + 2) * (b2 + 2) > 10 * 18) continue;
+                const long long t0 = (m0 + b0 - 1) / b0, t1 = (n1 + b1 - 1) / b1, t2 = (n2 + b2 - 1) / b2;
+                const double tiles = (double)t0 * t1 * t2;
+                const double staged = (double)b0 * b1 * b2 + 2.0 * b1 * b2 + 2.0 * b0 * b1 + (D == 3 ? 2.0 * b0 * b2 : 0.0);
+                const double waves = shared ? tiles : std::max(1.0, tiles / (148.0 * 2));
+                const double cost = waves * (staged + 128.0 + 60.0);
+                if (cost < bc) {
+                    bc = cost;
+                    best.b[0] = b0;
+                    best.b[1] = b1;
+                    best.b[2] = b2;
+                    best.t[0] = (int)t0;
+                    best.t[1] = (int)t1;
+                    best.t[2] = (int)t2;
+                }
+            }
+    best.ncell = best.b[0] * best.b[1] * best.b[2];
+    memo.D = D;
+    memo.m0 = m0;
+    memo.n1 = n1;
+    memo.n2 = n2;
+    memo.shared = shared;
+    memo.t = best;
+    best.s0 = s0;
+    return best;
+}
+
+}  // namespace bosss

@@ -1634,7 +1634,7 @@ int bosss_b200_xdg_create(const bosss_op_desc* opA, const bosss_op_desc* opB, co
             X->sb[0] = (b0 / P) * P;
             X->sb[1] = std::min(J, ((b1 + P - 1) / P) * P);
             bosss_options sopt = hopt;
-            sopt.kernel = 2;
+            sopt.kernel = hopt.kernel == 0 ? 0 : 2;   // automatic: modal (constant mu) or slab
             if (X->sb[1] - X->sb[0] < J && bosss_b200_create(opB, grid, &sopt, &X->hs) != BOSSS_OK) X->hs = nullptr;
         }
     }
