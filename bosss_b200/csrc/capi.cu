@@ -23,6 +23,7 @@
 #include "bsr.h"
 #include "handle.h"
 #include "modal.h"
+#include "sip.h"
 #include "faces_euler.h"
 #include "tc_volume.h"
 
@@ -111,7 +112,7 @@ static void legendre(int K, long double x, long double* L, long double* dL) {
     }
 }
 
-static void build_tables(int K, int Q, Tables1D& t) {
+void build_tables(int K, int Q, Tables1D& t) {
     std::memset(&t, 0, sizeof(t));
     double x[QMAX], w[QMAX];
     gauss_rule(Q, x, w);
@@ -552,7 +553,11 @@ int bosss_b200_create(const bosss_op_desc* op, const bosss_grid_desc* grid, cons
     for (int m = 0; m < 3; ++m) {
         // linear constant-coefficient scalar forms with an exact rule: the modal stencil kernel
         if (want == 0 && prec == BOSSS_PRECISION_FP64 && modal_applies(phys, ph, K, Q)) mode_variant[m] = VARIANT_MODAL;
+        // nonlinear diffusion in 3D: the face-once block kernel
+        else if (want == 0 && prec == BOSSS_PRECISION_FP64 && phys == PHYS_SIP && D == 3 && sip_entry(K, Q, m).launch)
+            mode_variant[m] = VARIANT_SIP;
         h->kern[m] = mode_variant[m] == VARIANT_MODAL ? modal_entry(phys, D, K, m)
+                     : mode_variant[m] == VARIANT_SIP ? sip_entry(K, Q, m)
                                                       : reg[KernelKey(phys, D, K, Q, m, mode_variant[m])];
         h->kern_variant[m] = mode_variant[m];
         if (mode_variant[m] == VARIANT_SLAB) h->variant = VARIANT_SLAB;
@@ -737,7 +742,9 @@ int bosss_b200_kernel_info(const bosss_handle* h, int32_t mode, int32_t* kernel,
     const bool split = mode == MODE_RES && h->precision == BOSSS_PRECISION_SPLIT_FP32;
     const bool once = h->faces_once && (mode == MODE_RES || mode == MODE_VJP);
     const bool slab = h->kern_variant[mode] == VARIANT_SLAB;
-    int k = slab ? 2 : (h->kern_variant[mode] == VARIANT_MODAL ? 5 : 1), n = 1;
+    int k = slab ? 2 : 1, n = 1;
+    if (h->kern_variant[mode] == VARIANT_MODAL) k = 5;
+    if (h->kern_variant[mode] == VARIANT_SIP) k = 6;
     if (split) {
         k = 4;
         n = once ? 3 : 2;

@@ -1,0 +1,108 @@
+// sip.cu -- instances and launches of the nonlinear-diffusion block kernel.
+#include "sip.h"
+
+#include <algorithm>
+
+#include "sip_kernel.cuh"
+
+namespace bosss {
+
+namespace {
+
+// block extents: every launch covers the cells [cbeg, cend); cost = waves of resident CTAs times the
+// phases of a block (staged cells, faces, volume), the faces between blocks being evaluated twice
+template <class C>
+ModalTile sip_tiling(const EvalArgs& a) {
+    const GridConst& g = a.g;
+    const bool rev = g.stride[0] == 1 && g.stride[2] != 1;
+    const int n0 = rev ? g.n[2] : g.n[0], n1 = g.n[1], n2 = rev ? g.n[0] : g.n[2];
+    const long long plane = (long long)n1 * n2;
+    const int s0 = (int)(a.cbeg / plane), s1 = (int)std::min<long long>(n0, (a.cend + plane - 1) / plane);
+    const int m0 = std::max(1, s1 - s0);
+    ModalTile best{};
+    double bc = 1e300;
+    const int ext[] = {1, 2, 3, 4, 5, 6, 8};
+    for (int b0 : ext)
+        for (int b1 : ext)
+            for (int b2 : ext) {
+                const int cells = b0 * b1 * b2;
+                const int fmax = cells + std::max(b1 * b2, std::max(b0 * b2, b0 * b1));
+                if (cells > C::CELLS || (b0 + 2) * (b1 + 2) * (b2 + 2) > C::SLOTS || fmax > C::FACES) continue;
+                const long long t0 = (m0 + b0 - 1) / b0, t1 = (n1 + b1 - 1) / b1, t2 = (n2 + b2 - 1) / b2;
+                const double tiles = (double)t0 * t1 * t2, slots = 148.0 * C::MINB;
+                const double faces = 3.0 * cells + b1 * b2 + b0 * b2 + b0 * b1;
+                // a CTA's time: fixed part (staging latency, barriers) + its work over its threads
+                const double cta = 40.0 + cells * 1.0 + faces * 0.8;
+                const double waves = tiles <= slots ? 1.0 : tiles / slots;
+                const double cost = waves * cta;
+                if (cost < bc) {
+                    bc = cost;
+                    best.b[0] = b0;
+                    best.b[1] = b1;
+                    best.b[2] = b2;
+                    best.t[0] = (int)t0;
+                    best.t[1] = (int)t1;
+                    best.t[2] = (int)t2;
+                }
+            }
+    best.s0 = s0;
+    best.ncell = best.b[0] * best.b[1] * best.b[2];
+    return best;
+}
+
+template <int K, int Q, int MODE>
+cudaError_t launch_sip(const EvalArgs& a, cudaStream_t s) {
+    using C = SipCfg<K, Q, MODE>;
+    if (a.vol_flag || a.face_flag) {   // species masks: the slab tile reads them
+        auto it = kernel_registry().find(KernelKey(PHYS_SIP, 3, K, Q, MODE, VARIANT_SLAB));
+        if (it == kernel_registry().end()) return cudaErrorNotSupported;
+        return it->second.launch(a, s);
+    }
+    static const Tables1D V = [] {
+        Tables1D t;
+        build_tables(K, C::QV, t);
+        return t;
+    }();
+    static unsigned long long done = 0ull;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (!(done & (1ull << (dev & 63)))) {
+        cudaError_t e = cudaFuncSetAttribute(k_sip<K, Q, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sip<K, Q, MODE>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        if (e != cudaSuccess) return e;
+        done |= 1ull << (dev & 63);
+    }
+    if (a.cend <= a.cbeg) return cudaSuccess;
+    const ModalTile tl = sip_tiling<C>(a);
+    k_sip<K, Q, MODE><<<tl.t[0] * tl.t[1] * tl.t[2], C::NT, C::SMEM, s>>>(a, V, tl);
+    return cudaGetLastError();
+}
+
+template <int K, int Q>
+KernelEntry entry_of(int mode) {
+    KernelEntry e{nullptr, SipCfg<K, Q, MODE_RES>::CELLS, SipCfg<K, Q, MODE_RES>::SMEM};
+    e.launch = mode == MODE_RES ? &launch_sip<K, Q, MODE_RES> : mode == MODE_JVP ? &launch_sip<K, Q, MODE_JVP> : &launch_sip<K, Q, MODE_VJP>;
+    return e;
+}
+
+}  // namespace
+
+KernelEntry sip_entry(int K, int Q, int mode) {
+#define BOSSS_SIP_CASE(k, q) \
+    if (K == k && Q == q) return entry_of<k, q>(mode);
+    BOSSS_SIP_CASE(1, 2)
+    BOSSS_SIP_CASE(1, 3)
+    BOSSS_SIP_CASE(2, 3)
+    BOSSS_SIP_CASE(2, 4)
+    BOSSS_SIP_CASE(2, 5)
+    BOSSS_SIP_CASE(3, 4)
+    BOSSS_SIP_CASE(3, 5)
+    BOSSS_SIP_CASE(3, 7)
+    BOSSS_SIP_CASE(4, 5)
+    BOSSS_SIP_CASE(4, 7)
+    BOSSS_SIP_CASE(4, 9)
+#undef BOSSS_SIP_CASE
+    return KernelEntry{nullptr, 0, 0};
+}
+
+}  // namespace bosss

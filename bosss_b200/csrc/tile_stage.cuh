@@ -1,0 +1,97 @@
+// tile_stage.cuh -- blocks of cells with a face halo in shared memory (scalar and system tiles).
+//
+// A CTA owns a block of b[0] x b[1] x b[2] cells in memory order (slow, middle, fast direction of
+// the local cell numbering). Every cell of the block and of its six face halos has a slot of S
+// doubles in a (b+2)^3 halo box; the corners stay unused. The copies are asynchronous 8-byte
+// ones: the caller's vectors may start at any double.
+#pragma once
+#include "modal.h"
+
+namespace bosss {
+
+__device__ __forceinline__ void tile_cp8(void* dst, const void* src) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void tile_cp_wait() {
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+}
+
+// memory-order view of a three-dimensional grid and the block of one tile
+struct TileGeom {
+    bool rev;          // GlobalID order: x fastest
+    int n[3], per[3];  // cells and periodicity per memory direction
+    int o[3], e[3];    // first cell and (clipped) extent of the block
+    int q0, q1;        // slot strides (in slots) of the slow and middle direction
+    __device__ __forceinline__ int slot(int i0, int i1, int i2) const { return (i0 + 1) * q0 + (i1 + 1) * q1 + i2 + 1; }
+    // memory direction of physical direction d
+    __device__ __forceinline__ int mem(int d) const { return rev ? 2 - d : d; }
+};
+
+__device__ __forceinline__ TileGeom tile_geom(const GridConst& g, const ModalTile& tl, int tile) {
+    TileGeom G;
+    G.rev = g.stride[0] == 1 && g.stride[2] != 1;
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+        G.n[m] = G.rev ? g.n[2 - m] : g.n[m];
+        G.per[m] = G.rev ? g.periodic[2 - m] : g.periodic[m];
+    }
+    const int t2 = tile % tl.t[2], tq = tile / tl.t[2];
+    const int t1 = tq % tl.t[1], t0 = tq / tl.t[1];
+    G.o[0] = tl.s0 + t0 * tl.b[0];
+    G.o[1] = t1 * tl.b[1];
+    G.o[2] = t2 * tl.b[2];
+#pragma unroll
+    for (int m = 0; m < 3; ++m) G.e[m] = min(tl.b[m], G.n[m] - G.o[m]);
+    G.q1 = tl.b[2] + 2;
+    G.q0 = (tl.b[1] + 2) * (tl.b[2] + 2);
+    return G;
+}
+
+// stage NC consecutive doubles per cell of `in` (cell-major) into slots of S doubles
+template <int NC, int S, int NT>
+__device__ __forceinline__ void tile_stage(const TileGeom& G, const double* __restrict__ in, double* sm) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int nw = NT >> 5;
+    const int rA = G.e[0] * G.e[1], rB = 2 * G.e[1], rC = 2 * G.e[0];
+    for (int r = warp; r < rA + rB + rC; r += nw) {
+        int i0, i1, f0 = 0, nf = G.e[2];
+        if (r < rA) {
+            i0 = r / G.e[1];
+            i1 = r - i0 * G.e[1];
+            f0 = -1;
+            nf = G.e[2] + 2;
+        } else if (r < rA + rB) {
+            const int q = r - rA;
+            i0 = (q & 1) ? G.e[0] : -1;
+            i1 = q >> 1;
+        } else {
+            const int q = r - rA - rB;
+            i0 = q >> 1;
+            i1 = (q & 1) ? G.e[1] : -1;
+        }
+        int m0 = G.o[0] + i0, m1 = G.o[1] + i1;
+        if (m0 < 0 || m0 >= G.n[0]) {
+            if (!G.per[0]) continue;
+            m0 = m0 < 0 ? m0 + G.n[0] : m0 - G.n[0];
+        }
+        if (m1 < 0 || m1 >= G.n[1]) {
+            if (!G.per[1]) continue;
+            m1 = m1 < 0 ? m1 + G.n[1] : m1 - G.n[1];
+        }
+        const long long row = ((long long)m0 * G.n[1] + m1) * G.n[2];
+        double* dst = sm + G.slot(i0, i1, 0) * S;
+        for (int e = lane; e < nf * NC; e += 32) {
+            const int c = e / NC, k = e - c * NC;
+            const int i2 = f0 + c;
+            int m2 = G.o[2] + i2;
+            if (m2 < 0 || m2 >= G.n[2]) {
+                if (!G.per[2]) continue;
+                m2 = m2 < 0 ? m2 + G.n[2] : m2 - G.n[2];
+            }
+            tile_cp8(dst + i2 * S + k, in + (row + m2) * NC + k);
+        }
+    }
+}
+
+}  // namespace bosss

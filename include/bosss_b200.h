@@ -202,8 +202,9 @@ int bosss_b200_get_sizes(const bosss_handle* h, int64_t* n_domain_dofs, int64_t*
 /* The kernel path in effect for `mode` (0 residual, 1 JVP, 2 VJP): 1 generic fused kernel,
  * 2 slab kernel, 3 slab volume pass + face-once face kernels, 4 tensor-core volume kernel +
  * face terms (split-precision residual), 5 modal stencil kernel (scalar operators, linear with
- * constant coefficients, rule exact for them; automatic choice only); and the kernel launches of
- * one whole-grid call. */
+ * constant coefficients, rule exact for them; automatic choice only), 6 face-once block kernel
+ * of nonlinear SIP diffusion in 3D (automatic choice only); and the kernel launches of one
+ * whole-grid call. */
 int bosss_b200_kernel_info(const bosss_handle* h, int32_t mode, int32_t* kernel, int32_t* launches);
 
 /* EvaluatorNonLin.Evaluate (DifferentialOperator.cs:1584-1661):
