@@ -22,6 +22,7 @@
 #include "dg_registry.h"
 #include "bsr.h"
 #include "handle.h"
+#include "euler_block.h"
 #include "modal.h"
 #include "sip.h"
 #include "faces_euler.h"
@@ -556,8 +557,14 @@ int bosss_b200_create(const bosss_op_desc* op, const bosss_grid_desc* grid, cons
         // nonlinear diffusion in 3D: the face-once block kernel
         else if (want == 0 && prec == BOSSS_PRECISION_FP64 && phys == PHYS_SIP && D == 3 && sip_entry(K, Q, m).launch)
             mode_variant[m] = VARIANT_SIP;
+        // Euler on periodic grids: the face-once block kernel (split-precision handles: the residual
+        // keeps the tensor-core volume and slab faces)
+        else if (want == 0 && (prec == BOSSS_PRECISION_FP64 || m != MODE_RES) && phys == PHYS_EULER && D == 3 && !euler_bounded &&
+                 euler_block_entry(K, Q, m).launch)
+            mode_variant[m] = VARIANT_EULER_BLOCK;
         h->kern[m] = mode_variant[m] == VARIANT_MODAL ? modal_entry(phys, D, K, m)
                      : mode_variant[m] == VARIANT_SIP ? sip_entry(K, Q, m)
+                     : mode_variant[m] == VARIANT_EULER_BLOCK ? euler_block_entry(K, Q, m)
                                                       : reg[KernelKey(phys, D, K, Q, m, mode_variant[m])];
         h->kern_variant[m] = mode_variant[m];
         if (mode_variant[m] == VARIANT_SLAB) h->variant = VARIANT_SLAB;
@@ -745,6 +752,7 @@ int bosss_b200_kernel_info(const bosss_handle* h, int32_t mode, int32_t* kernel,
     int k = slab ? 2 : 1, n = 1;
     if (h->kern_variant[mode] == VARIANT_MODAL) k = 5;
     if (h->kern_variant[mode] == VARIANT_SIP) k = 6;
+    if (h->kern_variant[mode] == VARIANT_EULER_BLOCK) k = 7;
     if (split) {
         k = 4;
         n = once ? 3 : 2;

@@ -505,7 +505,7 @@ class Evaluator:
     def kernel_info(self, mode=C.MODE_RESIDUAL):
         """(kernel path, launches per whole-grid call) of `mode`: 1 generic, 2 slab, 3 slab
         volume pass + face-once face kernels, 4 tensor-core volume + face terms, 5 modal stencil,
-        6 nonlinear-SIP blocks."""
+        6 nonlinear-SIP blocks, 7 Euler blocks."""
         k, n = ctypes.c_int32(), ctypes.c_int32()
         C.check(C.lib().bosss_b200_kernel_info(self.handle, int(mode), ctypes.byref(k), ctypes.byref(n)))
         return k.value, n.value
