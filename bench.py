@@ -793,7 +793,8 @@ def run_partitioned(args, rank, world, local):
 PATH_KERNELS = {1: "dg_cell_kernel<PhysEuler<3>,K,Q,%s>",
                 2: "dg_slab_kernel<PhysEuler<3>,K,Q,%s>",
                 3: "dg_slab_kernel<PhysEuler<3>,K,Q,%s> volume pass + k_euler_faces + k_euler_face_project",
-                4: "tc_volume_kernel + %s face terms"}
+                4: "tc_volume_kernel + %s face terms",
+                7: "k_euler_block<K,%s>"}
 
 
 def main():

@@ -9,10 +9,10 @@ namespace bosss {
 namespace {
 
 template <int D, int K, bool SIP, int MODE, bool MASK>
-__global__ void __launch_bounds__(MODAL_NT, ModalCfg<D, K>::MINB)
+__global__ void __launch_bounds__(ModalCfg<D, K>::NT, ModalCfg<D, K>::MINB)
 k_modal(const __grid_constant__ EvalArgs a, const __grid_constant__ ModalTile tl) {
     extern __shared__ double smem[];
-    modal_tile<D, K, SIP, MODE, MASK>(a, tl, blockIdx.x, MODE == MODE_RES ? a.U : a.V, a.out, a.alpha, a.beta, smem);
+    modal_tile<D, K, SIP, MODE, MASK>(a, a.tab, tl, blockIdx.x, MODE == MODE_RES ? a.U : a.V, a.out, a.alpha, a.beta, smem);
 }
 
 template <int D, int K, bool SIP, int MODE, bool MASK>
@@ -23,7 +23,7 @@ cudaError_t launch_masked(const EvalArgs& a, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     if (a.cend <= a.cbeg) return cudaSuccess;
     const ModalTile tl = modal_tiling(a, D, K);
-    k_modal<D, K, SIP, MODE, MASK><<<tl.t[0] * tl.t[1] * tl.t[2], MODAL_NT, smem, s>>>(a, tl);
+    k_modal<D, K, SIP, MODE, MASK><<<tl.t[0] * tl.t[1] * tl.t[2], ModalCfg<D, K>::NT, smem, s>>>(a, tl);
     return cudaGetLastError();
 }
 
@@ -37,7 +37,7 @@ cudaError_t launch_modal(const EvalArgs& a, cudaStream_t s) {
 
 template <int D, int K, bool SIP>
 KernelEntry entry_of(int mode) {
-    KernelEntry e{nullptr, MODAL_NT, ModalCfg<D, K>::SMEM};
+    KernelEntry e{nullptr, MODAL_CELLS, ModalCfg<D, K>::SMEM};
     e.launch = mode == MODE_RES   ? &launch_modal<D, K, SIP, MODE_RES>
                : mode == MODE_JVP ? &launch_modal<D, K, SIP, MODE_JVP>
                                   : &launch_modal<D, K, SIP, MODE_VJP>;
@@ -97,7 +97,7 @@ ModalTile modal_tiling(const EvalArgs& a, int D, int K, bool shared) {
         for (int b1 : c0)
             for (int b2 : c2) {
                 if (D == 2 && b1 != 1) continue;
-                if (b0 * b1 * b2 > MODAL_NT) continue;
+                if (b0 * b1 * b2 > MODAL_CELLS) continue;
                 if (D == 3 && (b0 + 2) * (b1 + 2) * (b2 + 2) > 6 * 6 * 10) continue;
                 if (D == 2 && (b0 + 2) * (b2 + 2) > 10 * 18) continue;
                 const long long t0 = (m0 + b0 - 1) / b0, t1 = (n1 + b1 - 1) / b1, t2 = (n2 + b2 - 1) / b2;

@@ -18,48 +18,48 @@ struct ModalInst {
 namespace {
 
 template <int K, bool SIP, int MODE>
-__global__ void __launch_bounds__(MODAL_NT, ModalCfg<3, K>::MINB)
-k_modal_batch(const ModalInst* __restrict__ inst, const ModalItem* __restrict__ items, const double* U, const double* V,
+__global__ void __launch_bounds__(ModalCfg<3, K>::NT, ModalCfg<3, K>::MINB)
+k_modal_batch(const __grid_constant__ Tables1D tab, const ModalInst* __restrict__ inst, const ModalItem* __restrict__ items, const double* U, const double* V,
               double* out, double alpha, double beta) {
     extern __shared__ double smem[];
     __shared__ ModalInst si;
     const ModalItem w = items[blockIdx.x];
     static_assert(sizeof(ModalInst) % 8 == 0, "copied as doubles");
-    for (int i = threadIdx.x; i < (int)(sizeof(ModalInst) / 8); i += MODAL_NT)
+    for (int i = threadIdx.x; i < (int)(sizeof(ModalInst) / 8); i += ModalCfg<3, K>::NT)
         reinterpret_cast<double*>(&si)[i] = reinterpret_cast<const double*>(inst + w.inst)[i];
     __syncthreads();
     const double* in = MODE == MODE_RES ? U + si.dom_off : V + (MODE == MODE_VJP ? si.cod_off : si.dom_off);
     double* o = out + (MODE == MODE_VJP ? si.dom_off : si.cod_off);
-    modal_tile<3, K, SIP, MODE, false>(si.a, si.tl, w.tile, in, o, alpha, beta, smem);
+    modal_tile<3, K, SIP, MODE, false>(si.a, tab, si.tl, w.tile, in, o, alpha, beta, smem);
 }
 
 template <int K, bool SIP, int MODE>
-cudaError_t launch_one(const ModalInst* inst, const ModalItem* items, int n, const double* U, const double* V,
+cudaError_t launch_one(const Tables1D& tab, const ModalInst* inst, const ModalItem* items, int n, const double* U, const double* V,
                        double* out, double alpha, double beta, cudaStream_t s) {
     static unsigned long long done = 0ull;
     const size_t smem = ModalCfg<3, K>::SMEM;
     cudaError_t e = modal_attr(k_modal_batch<K, SIP, MODE>, smem, done);
     if (e != cudaSuccess || n <= 0) return e;
-    k_modal_batch<K, SIP, MODE><<<n, MODAL_NT, smem, s>>>(inst, items, U, V, out, alpha, beta);
+    k_modal_batch<K, SIP, MODE><<<n, ModalCfg<3, K>::NT, smem, s>>>(tab, inst, items, U, V, out, alpha, beta);
     return cudaGetLastError();
 }
 
 template <int K, bool SIP>
-cudaError_t launch_mode(int mode, const ModalInst* inst, const ModalItem* items, int n, const double* U, const double* V,
+cudaError_t launch_mode(int mode, const Tables1D& tab, const ModalInst* inst, const ModalItem* items, int n, const double* U, const double* V,
                         double* out, double alpha, double beta, cudaStream_t s) {
-    if (mode == MODE_RES) return launch_one<K, SIP, MODE_RES>(inst, items, n, U, V, out, alpha, beta, s);
-    if (mode == MODE_JVP) return launch_one<K, SIP, MODE_JVP>(inst, items, n, U, V, out, alpha, beta, s);
-    return launch_one<K, SIP, MODE_VJP>(inst, items, n, U, V, out, alpha, beta, s);
+    if (mode == MODE_RES) return launch_one<K, SIP, MODE_RES>(tab, inst, items, n, U, V, out, alpha, beta, s);
+    if (mode == MODE_JVP) return launch_one<K, SIP, MODE_JVP>(tab, inst, items, n, U, V, out, alpha, beta, s);
+    return launch_one<K, SIP, MODE_VJP>(tab, inst, items, n, U, V, out, alpha, beta, s);
 }
 
 template <bool SIP>
-cudaError_t launch_degree(int K, int mode, const ModalInst* inst, const ModalItem* items, int n, const double* U,
+cudaError_t launch_degree(int K, int mode, const Tables1D& tab, const ModalInst* inst, const ModalItem* items, int n, const double* U,
                           const double* V, double* out, double alpha, double beta, cudaStream_t s) {
     switch (K) {
-        case 1: return launch_mode<1, SIP>(mode, inst, items, n, U, V, out, alpha, beta, s);
-        case 2: return launch_mode<2, SIP>(mode, inst, items, n, U, V, out, alpha, beta, s);
-        case 3: return launch_mode<3, SIP>(mode, inst, items, n, U, V, out, alpha, beta, s);
-        default: return launch_mode<4, SIP>(mode, inst, items, n, U, V, out, alpha, beta, s);
+        case 1: return launch_mode<1, SIP>(mode, tab, inst, items, n, U, V, out, alpha, beta, s);
+        case 2: return launch_mode<2, SIP>(mode, tab, inst, items, n, U, V, out, alpha, beta, s);
+        case 3: return launch_mode<3, SIP>(mode, tab, inst, items, n, U, V, out, alpha, beta, s);
+        default: return launch_mode<4, SIP>(mode, tab, inst, items, n, U, V, out, alpha, beta, s);
     }
 }
 
@@ -68,6 +68,7 @@ cudaError_t launch_degree(int K, int mode, const ModalInst* inst, const ModalIte
 struct ModalBatch {
     struct Run {
         int K, first, count;
+        Tables1D tab;   // of any instance of the degree (L_m(1), L_m'(1) depend on it alone)
     };
     bool sip = false;
     std::vector<Run> runs;   // highest degree first
@@ -98,9 +99,10 @@ int modal_batch_create(const std::vector<bosss_handle*>& hs, const long long* do
         inst[i].cod_off = cod_off[i];
     }
     for (int K = 4; K >= 1; --K) {
-        ModalBatch::Run r{K, (int)items.size(), 0};
+        ModalBatch::Run r{K, (int)items.size(), 0, Tables1D{}};
         for (size_t i = 0; i < hs.size(); ++i) {
             if (hs[i]->K != K) continue;
+            r.tab = hs[i]->base.tab;
             const ModalTile& t = inst[i].tl;
             for (int k = 0; k < t.t[0] * t.t[1] * t.t[2]; ++k) items.push_back(ModalItem{(int)i, k});
         }
@@ -122,8 +124,8 @@ int modal_batch_create(const std::vector<bosss_handle*>& hs, const long long* do
 int modal_batch_run(const ModalBatch* m, int mode, double alpha, double beta, const double* U, const double* V,
                     double* out, cudaStream_t s) {
     for (const auto& r : m->runs)
-        CUDA_TRY(m->sip ? launch_degree<true>(r.K, mode, m->d_inst, m->d_items + r.first, r.count, U, V, out, alpha, beta, s)
-                        : launch_degree<false>(r.K, mode, m->d_inst, m->d_items + r.first, r.count, U, V, out, alpha, beta, s));
+        CUDA_TRY(m->sip ? launch_degree<true>(r.K, mode, r.tab, m->d_inst, m->d_items + r.first, r.count, U, V, out, alpha, beta, s)
+                        : launch_degree<false>(r.K, mode, r.tab, m->d_inst, m->d_items + r.first, r.count, U, V, out, alpha, beta, s));
     return BOSSS_OK;
 }
 

@@ -18,11 +18,12 @@
 // necessary traffic per mode: HBM and FP64 pipe are within a factor of two of each other, where
 // the quadrature tiles spend 10-30x the arithmetic on node values.
 //
-// One thread per cell, both coefficient sets (input and result) in registers; a CTA's block of
-// cells and its face halo are staged in shared memory by asynchronous 8-byte copies (vectors
-// may start at any double), cells an odd number of doubles apart so that a warp reading the
-// same mode of 32 cells covers all banks. Results go back through the same slots, so that
-// global stores are runs of consecutive cells.
+// T threads per cell share the pencils of a direction (T by degree: a thread's chain of dependent
+// sums is what a small grid waits for, and short chains leave registers for more warps); the
+// three directions add to the cell's result in shared memory, each mode once per direction. A
+// CTA's block of cells and its face halo are staged by asynchronous 8-byte copies (vectors may
+// start at any double), cells an odd number of doubles apart so that a warp reading the same mode
+// of 32 cells covers all banks; results leave in runs of consecutive cells.
 //
 // Measured on B200 against the quadrature tiles: advection-diffusion 20x31x27 k = 3, residual + JVP +
 // VJP 495 -> 48 us; 16 instances of 16^3..32^3, k = 1..4, residual + VJP 3.69 -> 0.21 ms; XDG
@@ -33,22 +34,49 @@
 namespace bosss {
 
 
-static constexpr int MODAL_NT = 128;
-
-// sqrt((2m+1)/2) = L_m(1) and L_m'(1) = L_m(1) m (m+1) / 2
-__device__ constexpr double kE[5] = {0.70710678118654752440, 1.22474487139158904910, 1.58113883008418966600,
-                                     1.87082869338697069279, 2.12132034355964257320};
-// sqrt(2m+1)
-__device__ constexpr double kS[5] = {1.0, 1.73205080756887729353, 2.23606797749978969641, 2.64575131106459059050, 3.0};
+static constexpr int MODAL_CELLS = 128;   // cells of the largest tile
 
 template <int D, int K>
 struct ModalCfg {
     static constexpr int NP = np_of(D, K);
     static constexpr int S = NP | 1;                       // doubles per cell slot
-    // halo box of the largest tile: 4 x 4 x 8 cells in 3D, 8 x 16 in 2D, and one zero slot
+    static constexpr int PENCILS = D == 3 ? (K + 1) * (K + 2) / 2 : K + 1;
+    // threads per cell: the pencils of a direction are dealt to T threads
+    static constexpr int T = D == 2 ? 1 : (K == 4 ? 4 : K == 3 ? 2 : 1);
+    static constexpr int MINB = D == 2 ? 4 : (K == 4 ? 1 : K == 3 ? 2 : K == 2 ? 4 : 8);
+    static constexpr int NT = MODAL_CELLS * T;
+    // halo box of the largest tile: 4 x 4 x 8 cells in 3D, 8 x 16 in 2D, one zero slot, the results
     static constexpr int SLOTS = (D == 3 ? 6 * 6 * 10 : 10 * 18) + 1;
-    static constexpr size_t SMEM = sizeof(double) * S * SLOTS;
-    static constexpr int MINB = SMEM > 75 * 1024 ? 2 : (SMEM > 45 * 1024 ? 3 : 4);
+    // runs of cells to copy: per row of the tile its cells (with the halo cells that follow on), and
+    // halo cells across a periodic wrap; the rows of the slow and middle halos
+    static constexpr int ROWS = D == 3 ? 128 : 16, RUNS = 3 * ROWS;
+    static constexpr size_t SMEM = sizeof(double) * (S * (SLOTS + MODAL_CELLS) + 3 * 2 * 6);
+};
+struct ModalRun {
+    long long src;   // first double
+    int dst, n;      // slot offset, doubles
+};
+
+// thread (0 .. T-1) that evaluates pencil i = (p, r), r fastest: longest pencils first, each to the
+// least loaded thread
+template <int D, int K>
+struct PencilOwner {
+    int o[ModalCfg<D, K>::PENCILS] = {};
+    constexpr PencilOwner() {
+        int load[ModalCfg<D, K>::T] = {};
+        for (int L = K + 1; L >= 1; --L) {
+            int i = 0;
+            for (int p = 0; p <= K; ++p)
+                for (int r = 0; r <= (D == 3 ? K - p : 0); ++r, ++i) {
+                    if (K - p - r + 1 != L) continue;
+                    int best = 0;
+                    for (int t = 1; t < ModalCfg<D, K>::T; ++t)
+                        if (load[t] < load[best]) best = t;
+                    o[i] = best;
+                    load[best] += L + 2;
+                }
+        }
+    }
 };
 
 template <int D>
@@ -70,13 +98,225 @@ __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
 }
 
+// 1 / cell length scale of a cell (penalty_size without divisions)
+__device__ __forceinline__ double modal_size(const EvalArgs& a, const int* ijk) {
+    if (a.cell_pf) return penalty_size(a.cell_pf, a.g, ijk);
+    double cj = 0.0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        if (d >= a.g.D) break;
+        int nb = 2;
+        if (!a.g.gper[d]) {
+            const int gi = ijk[d] + a.g.goff[d];
+            nb += (gi == 0) + (gi == a.g.gn[d] - 1);
+        }
+        cj += nb * (0.5 * a.g.twoh[d]);
+    }
+    return 0.5 * cj;
+}
+
+// coefficients of face (dir, s) of cell ijk; nb: there is a neighbour whose coefficients enter
+template <int D, bool SIP, int MODE>
+__device__ __forceinline__ FaceCoef modal_face(const EvalArgs& a, const int* ijk, int dir, int s, bool on, bool& nb) {
+    const GridConst& g = a.g;
+    FaceCoef f{0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    const bool tr = a.ph.has_transport != 0, sip = SIP && a.ph.has_sip != 0;
+    const double th = g.twoh[dir], vel = tr ? a.ph.vel[dir] : 0.0, nu = sip ? a.ph.nu0 : 0.0;
+    int i = ijk[dir] + (s ? 1 : -1);
+    bool inner = true;
+    if (i < 0 || i >= g.n[dir]) {
+        inner = g.periodic[dir] != 0;
+        i = i < 0 ? i + g.n[dir] : i - g.n[dir];
+    }
+    nb = inner && on;
+    if (!on) return f;
+    if (inner) {
+        // upwind: the lower cell's value where vel > 0, else the upper cell's
+        const double ap = vel > 0.0 ? vel : 0.0, am = vel > 0.0 ? 0.0 : vel;
+        double p = 0.0;
+        if constexpr (SIP) {
+            int ijk2[3] = {ijk[0], ijk[1], ijk[2]};
+            ijk2[dir] = i;
+            p = sip ? a.ph.pen * fmax(modal_size(a, ijk), modal_size(a, ijk2)) * nu : 0.0;
+        }
+        if (MODE == MODE_VJP) {
+            f.p = p - (s ? ap : -am);   // both sides of the upwind flux see the jump of w
+        } else {
+            f.p = p;
+            f.cO = s ? ap : -am;
+            f.cN = s ? am : -ap;
+        }
+        f.hO = f.hN = 0.5 * nu * th;
+        f.k = 0.5 * nu;
+    } else {
+        const double an = s ? vel : -vel;
+        if (tr && (D == 2 || an >= 0.0)) f.cO = an;
+        if (sip && a.ph.dirichlet) {
+            f.p = 2.0 * a.ph.pen * modal_size(a, ijk) * nu;
+            f.hO = nu * th;
+            f.k = nu;
+        }
+    }
+    f.cO *= th;
+    f.cN *= th;
+    f.p *= th;
+    f.hO *= th;
+    f.hN *= th;
+    f.k *= th * th;
+    return f;
+}
+
+// the same between two cells that touch no boundary of the global grid
+template <int D, bool SIP, int MODE>
+__device__ __forceinline__ void modal_plain_face(const EvalArgs& a, int dir, int s, double* o) {
+    const bool tr = a.ph.has_transport != 0, sip = SIP && a.ph.has_sip != 0;
+    const double th = a.g.twoh[dir], vel = tr ? a.ph.vel[dir] : 0.0, nu = sip ? a.ph.nu0 : 0.0;
+    double cj = 0.0;
+#pragma unroll
+    for (int d = 0; d < D; ++d) cj += 2 * (0.5 * a.g.twoh[d]);
+    const double ap = vel > 0.0 ? vel : 0.0, am = vel > 0.0 ? 0.0 : vel;
+    const double p = sip ? a.ph.pen * (0.5 * cj) * nu : 0.0;
+    o[0] = MODE == MODE_VJP ? 0.0 : (s ? ap : -am) * th;
+    o[1] = MODE == MODE_VJP ? 0.0 : (s ? am : -ap) * th;
+    o[2] = (MODE == MODE_VJP ? p - (s ? ap : -am) : p) * th;
+    o[3] = o[4] = 0.5 * nu * th * th;
+    o[5] = 0.5 * nu * (th * th);
+}
+
+// the pencils of direction DIR that belong to thread TH of a cell: R (+)= their contributions
+template <int D, int K, bool SIP, int MODE, int DIR, int TH>
+__device__ __forceinline__ void modal_pencils(const Tables1D& T, const double* own, const double* nbu, const double* nbl,
+                                              const FaceCoef& fu, const FaceCoef& fl, double vT, double vS, double* R) {
+    constexpr PencilOwner<D, K> owner{};
+    constexpr int L1 = K + 1;
+    int i = 0;
+#pragma unroll
+    for (int p = 0; p <= K; ++p)
+#pragma unroll
+        for (int r = 0; r <= (D == 3 ? K - p : 0); ++r, ++i) {
+            if (owner.o[i] != TH) continue;
+            const int L = K - p - r + 1;
+            // own modes times L_m(1): w; with c_m = m (m+1) / 2 = L_m'(1) / L_m(1) everything on
+            // the pencil is sums of w and c w. L_m(-1) = (-1)^m L_m(1), L_m'(-1) = (-1)^(m+1) L_m'(1)
+            double w[L1], ue = 0.0, uo = 0.0, de = 0.0, dd = 0.0;
+            double x = 0.0, dx = 0.0, y = 0.0, dy = 0.0;
+#pragma unroll
+            for (int m = 0; m < L1; ++m)
+                if (m < L) {
+                    const int n = pencil_mode<D>(DIR, m, p, r);
+                    const double E = T.e[1][m], F = T.de[1][m], c = 0.5 * m * (m + 1);
+                    const double vu = nbu[n], vl = nbl[n];
+                    w[m] = own[n] * E;
+                    if (m & 1) uo += w[m];
+                    else ue += w[m];
+                    x += vu * ((m & 1) ? -E : E);
+                    y += vl * E;
+                    if (SIP && m > 0) {
+                        if (m & 1) dd += c * w[m];
+                        else de += c * w[m];
+                        dx += vu * ((m & 1) ? F : -F);
+                        dy += vl * F;
+                    }
+                }
+            const double uP = ue + uo, uM = ue - uo;
+            const double Ju = uP - x, Jl = uM - y;
+            double gu = fu.cO * uP - fu.p * Ju, gl = fl.cO * uM - fl.p * Jl, Gs = 0.0, Gd = 0.0;
+            if (MODE != MODE_VJP) {
+                gu += fu.cN * x;
+                gl += fl.cN * y;
+            }
+            if constexpr (SIP) {
+                gu += fu.hO * (de + dd) + fu.hN * dx;
+                gl -= fl.hO * (dd - de) + fl.hN * dy;
+                const double Gu = fu.k * Ju, Gl = fl.k * Jl;
+                Gs = Gu - Gl;
+                Gd = Gu + Gl;
+            }
+            const double gs = gu + gl, gd = gu - gl;
+            // volume: int L_a' L_m = 2 L_a(1) L_m(1) (m < a, a - m odd), int L_a' L_m' = 2 c_min L_a(1) L_m(1)
+            // (a - m even): sums over the modes below / above by parity
+            double pre[2] = {0.0, 0.0}, pc[2] = {0.0, 0.0}, up[2] = {ue, uo};
+#pragma unroll
+            for (int m = 0; m < L1; ++m)
+                if (m < L) {
+                    const int n = pencil_mode<D>(DIR, m, p, r);
+                    const double c = 0.5 * m * (m + 1);
+                    const int e = m & 1;
+                    up[e] -= w[m];   // modes above m of the same parity
+                    double h = e ? gd : gs;
+                    if (MODE == MODE_VJP) h += vT * up[1 - e];   // the other parity: those above m are left
+                    else h += vT * pre[1 - e];
+                    if (SIP && m > 0) {
+                        pc[e] += c * w[m];
+                        h += vS * pc[e] + c * ((e ? Gs : Gd) + vS * up[e]);
+                    }
+                    pre[e] += w[m];
+                    if (DIR == 0) R[n] = h * T.e[1][m];
+                    else R[n] += h * T.e[1][m];
+                }
+        }
+}
+
+// Dirichlet data of a boundary face (residual only): the trace of g_D on the modes of the face; g_D
+// is a sum of one-direction polynomials, so only p = 0 or r = 0 are non-zero
+template <int D, int K, int DIR>
+__device__ __forceinline__ void modal_boundary_data(const EvalArgs& a, const Tables1D& T, const int* ijk, int s,
+                                                    const FaceCoef& f, double* R) {
+    const GridConst& g = a.g;
+    constexpr int d1 = (DIR == 0) ? 1 : 0, d2 = (DIR == 2) ? 1 : 2;
+    const double xn = g.lo[DIR] + (ijk[DIR] + g.goff[DIR] + (s ? 1.0 : 0.0)) * g.h[DIR];
+    const double cst = a.ph.g0 + a.ph.g1[DIR] * xn + a.ph.g2[DIR] * xn * xn;
+    double M1[K + 1], M2[K + 1];
+#pragma unroll
+    for (int q = 0; q <= K; ++q) M1[q] = M2[q] = 0.0;
+    for (int q = 0; q < QMAX; ++q) {
+        const double w = a.tab.w[q];
+        if (w == 0.0) break;   // nodes of the rule (the rest of the table is zero)
+        const double x1 = g.lo[d1] + (ijk[d1] + g.goff[d1] + 0.5 + 0.5 * a.tab.xq[q]) * g.h[d1];
+        const double f1 = (a.ph.g1[d1] + a.ph.g2[d1] * x1) * x1 * w;
+        double f2 = 0.0;
+        if (D == 3) {
+            const double x2 = g.lo[d2] + (ijk[d2] + g.goff[d2] + 0.5 + 0.5 * a.tab.xq[q]) * g.h[d2];
+            f2 = (a.ph.g1[d2] + a.ph.g2[d2] * x2) * x2 * w;
+        }
+#pragma unroll
+        for (int p = 0; p <= K; ++p) {
+            M1[p] += f1 * a.tab.A[q][p];
+            if (D == 3) M2[p] += f2 * a.tab.A[q][p];
+        }
+    }
+    const double rt2 = 1.41421356237309504880, isc = 1.0 / g.scaling;
+#pragma unroll
+    for (int p = 0; p <= K; ++p)
+#pragma unroll
+        for (int r = 0; r <= (D == 3 ? K - p : 0); ++r) {
+            if (p > 0 && r > 0) continue;
+            double gD = M1[p] * ((D == 3) ? rt2 : 1.0);
+            if (r > 0) gD = 0.0;
+            if (D == 3 && p == 0) gD += M2[r] * rt2;
+            if (p == 0 && r == 0) gD += cst * ((D == 3) ? 2.0 : rt2);
+            gD *= isc;
+            const double gg = f.p * gD, GG = f.k * gD;
+#pragma unroll
+            for (int m = 0; m <= K - p - r; ++m) {
+                const int n = pencil_mode<D>(DIR, m, p, r);
+                const double E = T.e[1][m], F = T.de[1][m];
+                if (s) R[n] += gg * E - GG * F;
+                else R[n] += ((m & 1) ? -gg : gg) * E + ((m & 1) ? GG : -GG) * F;
+            }
+        }
+}
+
 // One tile: cells [o, o + b) in memory order (slow, middle, fast). MODE as the quadrature
-// kernels; MASK reads the species masks.
+// kernels; MASK reads the species masks. T: L_m(1) and L_m'(1) in T.e[1], T.de[1], in the
+// kernel-parameter bank so that they are operands of the FMAs (as literals they cost two moves
+// each: a third of all instructions of the first version).
 template <int D, int K, bool SIP, int MODE, bool MASK>
-__device__ __forceinline__ void modal_tile(const EvalArgs& a, const ModalTile& tl, int tile, const double* __restrict__ in,
-                                           double* __restrict__ out, double alpha, double beta, double* sm) {
+__device__ __forceinline__ void modal_tile(const EvalArgs& a, const Tables1D& T, const ModalTile& tl, int tile,
+                                           const double* __restrict__ in, double* __restrict__ out, double alpha, double beta,
+                                           double* sm) {
     using C = ModalCfg<D, K>;
-    constexpr int NP = C::NP, S = C::S;
+    constexpr int NP = C::NP, S = C::S, NT = C::NT;
     const GridConst& g = a.g;
     const int tid = threadIdx.x;
     // memory directions: generator order x slow .. z fast; GlobalID order the other way round
@@ -96,60 +336,71 @@ __device__ __forceinline__ void modal_tile(const EvalArgs& a, const ModalTile& t
         return ((i0 + 1) * q0 + ((D == 3) ? (i1 + 1) * q1 : 0) + (i2 + 1)) * S;
     };
     double* zero = sm + (C::SLOTS - 1) * S;
+    double* res = sm + C::SLOTS * S;
+    double* fct = res + MODAL_CELLS * S;   // [direction][side]: coefficients of a face between plain cells
     if (tid < NP) zero[tid] = 0.0;
 
-    // ---- stage the tile and its face halo: one warp per run of cells along the fast direction
-    {
-        const int warp = tid >> 5, lane = tid & 31, nw = MODAL_NT >> 5;
-        const int rA = e0 * e1, rB = 2 * e1, rC = (D == 3) ? 2 * e0 : 0;
-        for (int r = warp; r < rA + rB + rC; r += nw) {
-            int i0, i1, f0 = 0, nf = e2;
-            if (r < rA) {
-                i0 = r / e1;
-                i1 = r - i0 * e1;
-                f0 = -1;
-                nf = e2 + 2;
-            } else if (r < rA + rB) {
-                const int q = r - rA;
-                i0 = (q & 1) ? e0 : -1;
-                i1 = q >> 1;
-            } else {
-                const int q = r - rA - rB;
-                i0 = q >> 1;
-                i1 = (q & 1) ? e1 : -1;
-            }
-            int m0 = o0 + i0, m1 = o1 + i1;
-            if (m0 < 0 || m0 >= n0) {
-                if (!per0) continue;
-                m0 = m0 < 0 ? m0 + n0 : m0 - n0;
-            }
-            if (D == 3 && (m1 < 0 || m1 >= n1)) {
-                if (!per1) continue;
-                m1 = m1 < 0 ? m1 + n1 : m1 - n1;
-            }
-            const long long row = ((long long)m0 * n1 + m1) * n2;
-            double* dst = sm + slot(i0, i1, 0);
-            for (int e = lane; e < nf * NP; e += 32) {
-                const int c = e / NP, n = e - c * NP;
-                const int i2 = f0 + c;
-                int m2 = o2 + i2;
-                if (m2 < 0 || m2 >= n2) {
-                    if (!per2) continue;
-                    m2 = m2 < 0 ? m2 + n2 : m2 - n2;
-                }
-                cp_async8(dst + i2 * S + n, in + (row + m2) * NP + n);
-            }
+    // ---- stage the tile and its face halo: the runs of consecutive cells are found by one thread each
+    // (index arithmetic per row and warp took most of the time of the first version), then copied by
+    // the warps in turn
+    const int warp = tid >> 5, lane = tid & 31;
+    constexpr int nw = NT >> 5;
+    __shared__ ModalRun runs[C::RUNS];
+    const int rA = e0 * e1, rB = 2 * e1, rC = (D == 3) ? 2 * e0 : 0, nrows = rA + rB + rC;
+    for (int r = tid; r < nrows; r += NT) {
+        int i0, i1;
+        if (r < rA) {
+            i0 = r / e1;
+            i1 = r - i0 * e1;
+        } else if (r < rA + rB) {
+            i0 = ((r - rA) & 1) ? e0 : -1;
+            i1 = (r - rA) >> 1;
+        } else {
+            i0 = (r - rA - rB) >> 1;
+            i1 = ((r - rA - rB) & 1) ? e1 : -1;
         }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        int m0 = o0 + i0, m1 = o1 + i1;
+        bool there = true;
+        if (m0 < 0 || m0 >= n0) {
+            there = per0 != 0;
+            m0 = m0 < 0 ? m0 + n0 : m0 - n0;
+        }
+        if (D == 3 && (m1 < 0 || m1 >= n1)) {
+            there = there && per1 != 0;
+            m1 = m1 < 0 ? m1 + n1 : m1 - n1;
+        }
+        const long long row = ((long long)m0 * n1 + m1) * n2;
+        ModalRun main{(row + o2) * NP, slot(i0, i1, 0), there ? e2 * NP : 0}, lo{0, 0, 0}, hi{0, 0, 0};
+        if (r < rA) {
+            if (o2 > 0) {
+                main.src -= NP;
+                main.dst -= S;
+                main.n += NP;
+            } else if (per2) {
+                lo = ModalRun{(row + n2 - 1) * NP, slot(i0, i1, -1), NP};
+            }
+            if (o2 + e2 < n2) main.n += NP;
+            else if (per2) hi = ModalRun{row * NP, slot(i0, i1, e2), NP};
+        }
+        runs[3 * r] = main;
+        runs[3 * r + 1] = lo;
+        runs[3 * r + 2] = hi;
     }
+    __syncthreads();
+    for (int r = warp; r < 3 * nrows; r += nw) {
+        const ModalRun q = runs[r];
+        for (int e = lane; e < q.n; e += 32) cp_async8(sm + q.dst + e + (S - NP) * (e / NP), in + q.src + e);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
 
-    // ---- the thread's cell
-    const int l0 = tid / (b1 * b2), lr = tid - l0 * b1 * b2;
+    // ---- the thread's cell and share of the pencils
+    const int cell = tid % MODAL_CELLS, th = tid / MODAL_CELLS;   // th is warp-uniform
+    const int l0 = cell / (b1 * b2), lr = cell - l0 * b1 * b2;
     const int l1 = lr / b2, l2 = lr - l1 * b2;
     const int c0 = o0 + l0, c1 = o1 + l1, c2 = o2 + l2;
     const long long j = ((long long)c0 * n1 + c1) * n2 + c2;
     const bool active = l0 < e0 && l1 < e1 && l2 < e2 && j >= a.cbeg && j < a.cend;
-    int ijk[3] = {rev ? c2 : c0, (D == 3) ? c1 : c2, (D == 3) ? (rev ? c0 : c2) : 0};
+    const int ijk[3] = {rev ? c2 : c0, (D == 3) ? c1 : c2, (D == 3) ? (rev ? c0 : c2) : 0};
     double volm = 1.0;
     unsigned fmask = 0x3fu;
     if constexpr (MASK) {
@@ -162,240 +413,112 @@ __device__ __forceinline__ void modal_tile(const EvalArgs& a, const ModalTile& t
             }
         }
     }
+    const double* own = sm + (active ? slot(l0, l1, l2) : 0);
+    // a cell without any standard term takes no part (its coefficients may be anything)
+    if (MASK && volm == 0.0 && fmask == 0) own = zero;
+    double* R = res + cell * S;
+    // a face between two cells away from the boundaries of the global grid has the same
+    // coefficients everywhere (unless the caller gives length scales): computed once per CTA
+    if (tid < 2 * D) modal_plain_face<D, SIP, MODE>(a, tid >> 1, tid & 1, fct + tid * 6);
+    unsigned pl = 0;   // bits 2d, 2d + 1: own cell plain along d, and so is its lower / upper neighbour
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+        const int gi = ijk[d] + g.goff[d];
+        const bool p = g.gper[d] || (gi >= 1 && gi <= g.gn[d] - 2);
+        pl |= (p && (g.gper[d] || gi >= 2) ? 1u : 0u) << (2 * d) | (p && (g.gper[d] || gi <= g.gn[d] - 3) ? 2u : 0u) << (2 * d) |
+              (p ? 1u : 0u) << (8 + d);
+    }
+    const bool uniform = !SIP || !a.cell_pf;
+    const double nu0 = (SIP && a.ph.has_sip) ? a.ph.nu0 : 0.0;
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
 
-    double R[NP];
-#pragma unroll
-    for (int n = 0; n < NP; ++n) R[n] = 0.0;
-    if (active) {
-        const double* own = sm + slot(l0, l1, l2);
-        // a cell without any standard term takes no part (its coefficients may be anything)
-        if (MASK && volm == 0.0 && fmask == 0) own = zero;
-        double u[NP];
-#pragma unroll
-        for (int n = 0; n < NP; ++n) u[n] = own[n];
-        const bool tr = a.ph.has_transport != 0, sip = SIP && a.ph.has_sip != 0;
-        const double nu = sip ? a.ph.nu0 : 0.0;
-        double pfo = 0.0;
-        if (SIP) pfo = penalty_size(a.cell_pf, g, ijk);
-
-        auto direction = [&](auto dirc) {
-            constexpr int DIR = decltype(dirc)::value;
-            const double th = g.twoh[DIR], vel = tr ? a.ph.vel[DIR] : 0.0;
+    auto direction = [&](auto dirc) {
+        constexpr int DIR = decltype(dirc)::value;
+        if (active) {
+            const double thd = g.twoh[DIR], vel = a.ph.has_transport ? a.ph.vel[DIR] : 0.0;
             const int sl = (DIR == 0 ? (rev ? 1 : q0) : DIR == 1 ? (D == 3 ? q1 : 1) : (rev ? q0 : 1)) * S;
-            FaceCoef fu, fl;
-            const double *nbu = own + sl, *nbl = own - sl;
+            bool h[2];
+            FaceCoef fc[2];
+            constexpr unsigned others = (D == 3 ? 7u : 3u) & ~(1u << DIR);
 #pragma unroll
             for (int s = 0; s < 2; ++s) {
-                FaceCoef& f = s ? fu : fl;
-                const double*& nb = s ? nbu : nbl;
-                f = FaceCoef{0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-                int i = ijk[DIR] + (s ? 1 : -1);
-                bool inner = true;
-                if (i < 0 || i >= g.n[DIR]) {
-                    inner = g.periodic[DIR] != 0;
-                    i = i < 0 ? i + g.n[DIR] : i - g.n[DIR];
-                }
                 const bool on = !MASK || ((fmask >> (2 * DIR + s)) & 1u);
-                if (!inner || !on) nb = zero;
-                if (!on) continue;
-                if (inner) {
-                    // upwind: the lower cell's value where vel > 0, else the upper cell's
-                    const double ap = vel > 0.0 ? vel : 0.0, am = vel > 0.0 ? 0.0 : vel;
-                    double p = 0.0;
-                    if constexpr (SIP) {
-                        int ijk2[3] = {ijk[0], ijk[1], ijk[2]};
-                        ijk2[DIR] = i;
-                        p = sip ? a.ph.pen * fmax(pfo, penalty_size(a.cell_pf, g, ijk2)) * nu : 0.0;
-                    }
-                    if (MODE == MODE_VJP) {
-                        f.p = p - (s ? ap : -am);   // both sides of the upwind flux see the jump of w
-                    } else {
-                        f.p = p;
-                        f.cO = s ? ap : -am;
-                        f.cN = s ? am : -ap;
-                    }
-                    f.hO = f.hN = 0.5 * nu * th;
-                    f.k = 0.5 * nu;
+                const int i = ijk[DIR] + (s ? 1 : -1);
+                const bool inner = (i >= 0 && i < g.n[DIR]) || g.periodic[DIR];
+                const bool plain = !SIP || (uniform && ((pl >> (2 * DIR + s)) & 1u) && ((pl >> 8) & others) == others);
+                h[s] = inner && on;
+                if (h[s] && plain) {
+                    const double* q = fct + (2 * DIR + s) * 6;
+                    fc[s] = FaceCoef{q[0], q[1], q[2], q[3], q[4], q[5]};
                 } else {
-                    const double an = s ? vel : -vel;
-                    if (tr && (D == 2 || an >= 0.0)) f.cO = an;
-                    if (sip && a.ph.dirichlet) {
-                        const double p = 2.0 * a.ph.pen * pfo * nu;
-                        f.p = p;
-                        f.hO = nu * th;
-                        f.k = nu;
-                    }
+                    fc[s] = modal_face<D, SIP, MODE>(a, ijk, DIR, s, on, h[s]);
                 }
-                f.cO *= th;
-                f.cN *= th;
-                f.p *= th;
-                f.hO *= th;
-                f.hN *= th;
-                f.k *= th * th;
             }
-            const double vT = -vel * th * volm, vS = -nu * th * th * volm;
-#pragma unroll
-            for (int p = 0; p <= K; ++p)
-#pragma unroll
-                for (int r = 0; r <= (D == 3 ? K - p : 0); ++r) {
-                    constexpr int L1 = K + 1;
-                    const int L = K - p - r + 1;
-                    // traces: e = even, o = odd modes; L_m(-1) = (-1)^m L_m(1), L_m'(-1) = (-1)^(m+1) L_m'(1)
-                    double ue = 0.0, uo = 0.0, de = 0.0, dd = 0.0;
-                    double xe = 0.0, xo = 0.0, xde = 0.0, xdo = 0.0, y = 0.0, dy = 0.0;
-#pragma unroll
-                    for (int m = 0; m < L1; ++m)
-                        if (m < L) {
-                            const int n = pencil_mode<D>(DIR, m, p, r);
-                            const double E = kE[m], F = kE[m] * (0.5 * m * (m + 1));
-                            const double v = u[n], vu = nbu[n], vl = nbl[n];
-                            if (m & 1) {
-                                uo += v * E;
-                                xo += vu * E;
-                            } else {
-                                ue += v * E;
-                                xe += vu * E;
-                            }
-                            y += vl * E;
-                            if (SIP && m > 0) {
-                                if (m & 1) {
-                                    dd += v * F;
-                                    xdo += vu * F;
-                                } else {
-                                    de += v * F;
-                                    xde += vu * F;
-                                }
-                                dy += vl * F;
-                            }
-                        }
-                    const double uP = ue + uo, uM = ue - uo, x = xe - xo;
-                    const double Ju = uP - x, Jl = uM - y;
-                    double gu = fu.cO * uP - fu.p * Ju, gl = fl.cO * uM - fl.p * Jl, Gu = 0.0, Gl = 0.0;
-                    if (MODE != MODE_VJP) {
-                        gu += fu.cN * x;
-                        gl += fl.cN * y;
-                    }
-                    if constexpr (SIP) {
-                        const double dP = de + dd, dM = dd - de, dx = xdo - xde;
-                        gu += fu.hO * dP + fu.hN * dx;
-                        gl -= fl.hO * dM + fl.hN * dy;
-                        Gu = fu.k * Ju;
-                        Gl = -fl.k * Jl;
-                    }
-                    const double gs = gu + gl, gd = gu - gl, Gs = Gu + Gl, Gd = Gu - Gl;
-#pragma unroll
-                    for (int m = 0; m < L1; ++m)
-                        if (m < L) {
-                            const int n = pencil_mode<D>(DIR, m, p, r);
-                            const double E = kE[m], F = kE[m] * (0.5 * m * (m + 1));
-                            double t = R[n] + ((m & 1) ? gd : gs) * E;
-                            if (SIP && m > 0) t += ((m & 1) ? Gs : Gd) * F;
-                            // volume
-                            double tD = 0.0, tS = 0.0;
-#pragma unroll
-                            for (int q = 0; q < L1; ++q)
-                                if (q < L) {
-                                    const int nq = pencil_mode<D>(DIR, q, p, r);
-                                    const bool lower = (MODE == MODE_VJP) ? q > m : q < m;
-                                    if (lower && ((m - q) & 1)) tD += u[nq] * (kS[m] * kS[q]);
-                                    if (SIP && q > 0 && m > 0 && !((m - q) & 1)) {
-                                        const int mn = q < m ? q : m;
-                                        tS += u[nq] * (kS[m] * kS[q] * (0.5 * mn * (mn + 1)));
-                                    }
-                                }
-                            t += vT * tD;
-                            if (SIP && m > 0) t += vS * tS;
-                            R[n] = t;
-                        }
+            const bool hl = h[0], hu = h[1];
+            const FaceCoef &fl = fc[0], &fu = fc[1];
+            const double* nbu = hu ? own + sl : zero;
+            const double* nbl = hl ? own - sl : zero;
+            const double vT = -2.0 * vel * thd * volm, vS = -2.0 * nu0 * thd * thd * volm;
+            if constexpr (C::T == 1) {
+                modal_pencils<D, K, SIP, MODE, DIR, 0>(T, own, nbu, nbl, fu, fl, vT, vS, R);
+            } else {
+                if (th == 0) modal_pencils<D, K, SIP, MODE, DIR, 0>(T, own, nbu, nbl, fu, fl, vT, vS, R);
+                else if (th == 1) modal_pencils<D, K, SIP, MODE, DIR, 1>(T, own, nbu, nbl, fu, fl, vT, vS, R);
+                if constexpr (C::T > 2) {
+                    if (th == 2) modal_pencils<D, K, SIP, MODE, DIR, 2>(T, own, nbu, nbl, fu, fl, vT, vS, R);
                 }
-            // Dirichlet data of boundary faces (residual only): the trace of g_D on the modes of the
-            // face; g_D is a sum of one-direction polynomials, so only p = 0 or r = 0 are non-zero
-            if constexpr (SIP && MODE == MODE_RES) {
-                bool any = a.ph.g0 != 0.0;
+                if constexpr (C::T > 3) {
+                    if (th == 3) modal_pencils<D, K, SIP, MODE, DIR, 3>(T, own, nbu, nbl, fu, fl, vT, vS, R);
+                }
+            }
+        }
+        __syncthreads();
+    };
+    direction(std::integral_constant<int, 0>{});
+    direction(std::integral_constant<int, 1>{});
+    if constexpr (D == 3) direction(std::integral_constant<int, 2>{});
+
+    if constexpr (SIP && MODE == MODE_RES) {
+        bool any = a.ph.g0 != 0.0;
 #pragma unroll
-                for (int d = 0; d < D; ++d) any = any || a.ph.g1[d] != 0.0 || a.ph.g2[d] != 0.0;
-                if (any && sip && a.ph.dirichlet && !g.periodic[DIR]) {
+        for (int d = 0; d < D; ++d) any = any || a.ph.g1[d] != 0.0 || a.ph.g2[d] != 0.0;
+        const bool data = any && a.ph.has_sip && a.ph.dirichlet;
+        if (data || a.ph.has_source) {   // uniform over the CTA
+            if (active && th == 0) {
+                auto faces = [&](auto dirc) {
+                    constexpr int DIR = decltype(dirc)::value;
+                    if (!data || g.periodic[DIR]) return;
 #pragma unroll
                     for (int s = 0; s < 2; ++s) {
-                        const FaceCoef& f = s ? fu : fl;
                         if (ijk[DIR] != (s ? g.n[DIR] - 1 : 0)) continue;
                         if (MASK && !((fmask >> (2 * DIR + s)) & 1u)) continue;
-                        constexpr int d1 = (DIR == 0) ? 1 : 0, d2 = (DIR == 2) ? 1 : 2;
-                        const double xn = g.lo[DIR] + (ijk[DIR] + g.goff[DIR] + (s ? 1.0 : 0.0)) * g.h[DIR];
-                        const double cst = a.ph.g0 + a.ph.g1[DIR] * xn + a.ph.g2[DIR] * xn * xn;
-                        double M1[K + 1], M2[K + 1];
-#pragma unroll
-                        for (int q = 0; q <= K; ++q) M1[q] = M2[q] = 0.0;
-                        for (int q = 0; q < QMAX; ++q) {
-                            const double w = a.tab.w[q];
-                            if (w == 0.0) break;   // nodes of the rule (the rest of the table is zero)
-                            const double x1 = g.lo[d1] + (ijk[d1] + g.goff[d1] + 0.5 + 0.5 * a.tab.xq[q]) * g.h[d1];
-                            const double f1 = (a.ph.g1[d1] + a.ph.g2[d1] * x1) * x1 * w;
-                            double f2 = 0.0;
-                            if (D == 3) {
-                                const double x2 = g.lo[d2] + (ijk[d2] + g.goff[d2] + 0.5 + 0.5 * a.tab.xq[q]) * g.h[d2];
-                                f2 = (a.ph.g1[d2] + a.ph.g2[d2] * x2) * x2 * w;
-                            }
-#pragma unroll
-                            for (int p = 0; p <= K; ++p) {
-                                M1[p] += f1 * a.tab.A[q][p];
-                                if (D == 3) M2[p] += f2 * a.tab.A[q][p];
-                            }
-                        }
-                        const double rt2 = 1.41421356237309504880, isc = 1.0 / g.scaling;
-#pragma unroll
-                        for (int p = 0; p <= K; ++p)
-#pragma unroll
-                            for (int r = 0; r <= (D == 3 ? K - p : 0); ++r) {
-                                if (p > 0 && r > 0) continue;
-                                double gD = M1[p] * ((D == 3) ? rt2 : 1.0);
-                                if (r > 0) gD = 0.0;
-                                if (D == 3 && p == 0) gD += M2[r] * rt2;
-                                if (p == 0 && r == 0) gD += cst * ((D == 3) ? 2.0 : rt2);
-                                gD *= isc;
-                                const double gg = f.p * gD, GG = f.k * gD;
-#pragma unroll
-                                for (int m = 0; m <= K - p - r; ++m) {
-                                    const int n = pencil_mode<D>(DIR, m, p, r);
-                                    const double E = kE[m], F = kE[m] * (0.5 * m * (m + 1));
-                                    if (s) R[n] += gg * E - GG * F;
-                                    else R[n] += ((m & 1) ? -gg : gg) * E + ((m & 1) ? GG : -GG) * F;
-                                }
-                            }
+                        bool nb;
+                        const FaceCoef f = modal_face<D, SIP, MODE>(a, ijk, DIR, s, true, nb);
+                        modal_boundary_data<D, K, DIR>(a, T, ijk, s, f, R);
                     }
-                }
+                };
+                faces(std::integral_constant<int, 0>{});
+                faces(std::integral_constant<int, 1>{});
+                if constexpr (D == 3) faces(std::integral_constant<int, 2>{});
+                if (a.ph.has_source) R[0] += volm * a.ph.src * g.detJ * g.scaling * ((D == 3) ? 2.82842712474619009760 : 2.0);
             }
-        };
-        direction(std::integral_constant<int, 0>{});
-        direction(std::integral_constant<int, 1>{});
-        if constexpr (D == 3) direction(std::integral_constant<int, 2>{});
-        if (SIP && MODE == MODE_RES && a.ph.has_source)
-            R[0] += volm * a.ph.src * g.detJ * g.scaling * ((D == 3) ? 2.82842712474619009760 : 2.0);
+            __syncthreads();
+        }
     }
-    __syncthreads();
-    // ---- results through the cell's own slot, stored in runs of cells
-    if (active) {
-        double* own = sm + slot(l0, l1, l2);
-#pragma unroll
-        for (int n = 0; n < NP; ++n) own[n] = R[n];
-    }
-    __syncthreads();
-    {
-        const int warp = tid >> 5, lane = tid & 31, nw = MODAL_NT >> 5;
-        for (int r = warp; r < e0 * e1; r += nw) {
-            const int i0 = r / e1, i1 = r - i0 * e1;
-            const long long row = ((long long)(o0 + i0) * n1 + (o1 + i1)) * n2 + o2;
-            const double* src = sm + slot(i0, i1, 0);
-            for (int e = lane; e < e2 * NP; e += 32) {
-                const int c = e / NP;
-                if (row + c < a.cbeg || row + c >= a.cend) continue;
-                const double v = src[e + c * (S - NP)];
-                double* q = out + row * NP + e;
-                if (MODE == MODE_RES) *q = (beta == 0.0) ? alpha * v : beta * *q + alpha * v;
-                else *q = v;
-            }
+    // ---- results stored in runs of cells
+    for (int r = warp; r < e0 * e1; r += nw) {
+        const int i0 = r / e1, i1 = r - i0 * e1;
+        const long long row = ((long long)(o0 + i0) * n1 + (o1 + i1)) * n2 + o2;
+        const double* src = res + ((i0 * b1 + i1) * b2) * S;
+        double* dst = out + row * NP;
+        const bool whole = row >= a.cbeg && row + e2 <= a.cend;
+        for (int e = lane; e < e2 * NP; e += 32) {
+            const int c = e / NP;
+            if (!whole && (row + c < a.cbeg || row + c >= a.cend)) continue;
+            const double v = src[e + c * (S - NP)];
+            if (MODE == MODE_RES) dst[e] = (beta == 0.0) ? alpha * v : beta * dst[e] + alpha * v;
+            else dst[e] = v;
         }
     }
 }
