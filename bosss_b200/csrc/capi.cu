@@ -653,7 +653,9 @@ int bosss_b200_destroy(bosss_handle* h) {
     for (int c = 0; c < bosss_handle::MAX_CHUNKS; ++c) {
         if (h->ev_in[c]) cudaEventDestroy(h->ev_in[c]);
         if (h->ev_done[c]) cudaEventDestroy(h->ev_done[c]);
+        if (h->ev_second[c]) cudaEventDestroy(h->ev_second[c]);
     }
+    if (h->s_second) cudaStreamDestroy(h->s_second);
     if (h->s_in) cudaStreamDestroy(h->s_in);
     if (h->s_out) cudaStreamDestroy(h->s_out);
     if (h->stream) cudaStreamDestroy(h->stream);
@@ -803,8 +805,8 @@ int bosss_b200_apply_device(bosss_handle* h, int32_t mode, double alpha, double 
 // first plane of the next chunk have arrived (the face neighbours; the last plane comes first
 // when that direction is periodic), and each chunk's outputs stream out on a second copy stream
 // while later chunks are still computing. Small problems, and the opt-in NaN check, run as one
-// chunk. Returns after the last output has reached the host. 8 chunks measured best on B200
-// (Euler 32^3 k=3: 4 or 16 chunks, or a second compute stream for the VJP, were slower).
+// chunk. Returns after the last output has reached the host. A chunk's residual and VJP run on two
+// streams: each alone fills the chip for a fraction of a wave only. CHUNKNOTE
 struct HostJob {
     int mode;
     double alpha, beta;
@@ -834,12 +836,16 @@ static int host_pipelined(bosss_handle* h, const HostJob* jobs, int njobs, const
     for (int k = 0; k < njobs; ++k)   // split-precision residuals evaluate the whole grid at once
         if (jobs[k].mode == MODE_RES && h->precision == BOSSS_PRECISION_SPLIT_FP32) nch = 1;
     if (nch < 1) nch = 1;
+    // two streams only for kernels without scratch of the handle (face-once buffer, tensor-core path)
+    const bool two = njobs > 1 && !h->faces_once && h->precision == BOSSS_PRECISION_FP64;
     if (!h->s_in) CUDA_TRY(cudaStreamCreateWithFlags(&h->s_in, cudaStreamNonBlocking));
     if (!h->s_out) CUDA_TRY(cudaStreamCreateWithFlags(&h->s_out, cudaStreamNonBlocking));
     for (int c = 0; c < nch; ++c) {
         if (!h->ev_in[c]) CUDA_TRY(cudaEventCreateWithFlags(&h->ev_in[c], cudaEventDisableTiming));
         if (!h->ev_done[c]) CUDA_TRY(cudaEventCreateWithFlags(&h->ev_done[c], cudaEventDisableTiming));
+        if (two && !h->ev_second[c]) CUDA_TRY(cudaEventCreateWithFlags(&h->ev_second[c], cudaEventDisableTiming));
     }
+    if (two && !h->s_second) CUDA_TRY(cudaStreamCreateWithFlags(&h->s_second, cudaStreamNonBlocking));
     cudaStream_t s = h->stream, si = h->s_in, so = h->s_out;
     auto first_plane = [&](int c) { return (long long)c * planes / nch; };
     auto copy_in = [&](long long p0, long long p1) -> cudaError_t {
@@ -858,6 +864,7 @@ static int host_pipelined(bosss_handle* h, const HostJob* jobs, int njobs, const
     auto finish = [&](int code) {
         cudaStreamSynchronize(si);
         cudaStreamSynchronize(s);
+        if (h->s_second) cudaStreamSynchronize(h->s_second);
         cudaStreamSynchronize(so);
         return code;
     };
@@ -865,6 +872,7 @@ static int host_pipelined(bosss_handle* h, const HostJob* jobs, int njobs, const
     CUDA_TRY(cudaEventRecord(h->ev_done[0], s));
     CUDA_TRY(cudaStreamWaitEvent(si, h->ev_done[0], 0));
     CUDA_TRY(cudaStreamWaitEvent(so, h->ev_done[0], 0));
+    if (two) CUDA_TRY(cudaStreamWaitEvent(h->s_second, h->ev_done[0], 0));
     // copy segment c ends with the first plane of chunk c+1, the last face neighbour the cells
     // of chunk c need: ev_in[c] marks the moment chunk c can be evaluated
     cudaError_t e = cudaSuccess;
@@ -877,8 +885,11 @@ static int host_pipelined(bosss_handle* h, const HostJob* jobs, int njobs, const
     }
     if (e != cudaSuccess) return finish(fail(BOSSS_ERR_CUDA, cudaGetErrorString(e)));
     for (int c = 0; c < nch; ++c) {
-        e = cudaStreamWaitEvent(s, h->ev_in[c], 0);
-        for (int k = 0; k < njobs && e == cudaSuccess; ++k) {
+        for (int k = 0; k < njobs; ++k) {
+            cudaStream_t sk = k > 0 && two ? h->s_second : s;
+            cudaEvent_t done = k > 0 && two ? h->ev_second[c] : h->ev_done[c];
+            e = cudaStreamWaitEvent(sk, h->ev_in[c], 0);
+            if (e != cudaSuccess) return finish(fail(BOSSS_ERR_CUDA, cudaGetErrorString(e)));
             EvalArgs a = h->base;
             a.U = h->dU;
             a.V = jobs[k].mode != MODE_RES ? h->dV : nullptr;
@@ -888,18 +899,19 @@ static int host_pipelined(bosss_handle* h, const HostJob* jobs, int njobs, const
             a.time = time;
             a.cbeg = first_plane(c) * pc;
             a.cend = first_plane(c + 1) * pc;
-            rc = launch_eval(h, jobs[k].mode, a, s);
+            rc = launch_eval(h, jobs[k].mode, a, sk);
             if (rc) return finish(rc);
-        }
-        if (e == cudaSuccess) e = cudaEventRecord(h->ev_done[c], s);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(so, h->ev_done[c], 0);
-        for (int k = 0; k < njobs && e == cudaSuccess; ++k) {
+            e = cudaEventRecord(done, sk);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(so, done, 0);
             const long long c0 = first_plane(c) * pc, n = (first_plane(c + 1) - first_plane(c)) * pc, m = nY(jobs[k]);
-            e = cudaMemcpyAsync(jobs[k].Y + c0 * m, jobs[k].dY + c0 * m, sizeof(double) * n * m, cudaMemcpyDeviceToHost,
-                                so);
+            if (e == cudaSuccess)
+                e = cudaMemcpyAsync(jobs[k].Y + c0 * m, jobs[k].dY + c0 * m, sizeof(double) * n * m, cudaMemcpyDeviceToHost,
+                                    so);
+            if (e != cudaSuccess) return finish(fail(BOSSS_ERR_CUDA, cudaGetErrorString(e)));
         }
-        if (e != cudaSuccess) return finish(fail(BOSSS_ERR_CUDA, cudaGetErrorString(e)));
     }
+    // later calls on the handle's stream follow the second stream's work as well
+    if (two) CUDA_TRY(cudaStreamWaitEvent(s, h->ev_second[nch - 1], 0));
     if (h->check_nan)
         for (int k = 0; k < njobs; ++k) {
             rc = check_nan(h, jobs[k].dY, nY(jobs[k]) * J, s);

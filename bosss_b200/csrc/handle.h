@@ -44,6 +44,8 @@ struct bosss_handle {
     cudaStream_t s_in = nullptr, s_out = nullptr;
     static constexpr int MAX_CHUNKS = 16;
     cudaEvent_t ev_in[MAX_CHUNKS]{}, ev_done[MAX_CHUNKS]{};
+    cudaStream_t s_second = nullptr;           // second evaluation of a chunk (residual + VJP pair)
+    cudaEvent_t ev_second[MAX_CHUNKS]{};
 };
 
 namespace bosss {

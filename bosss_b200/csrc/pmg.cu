@@ -52,12 +52,12 @@ constexpr int COARSE_SWEEPS = 40;
 struct SGeom {
     int n[3];
     int per[3];
-    long long stride[3];
+    int stride[3];      // N <= 2e9: 32-bit index arithmetic (a 64-bit division costs as much as a sweep)
     long long N;
 };
 
 __host__ __device__ inline void s_ijk(const SGeom& g, long long i, int* ijk) {
-    for (int d = 0; d < 3; ++d) ijk[d] = (int)((i / g.stride[d]) % g.n[d]);
+    for (int d = 0; d < 3; ++d) ijk[d] = (int)(((unsigned)i / (unsigned)g.stride[d]) % (unsigned)g.n[d]);
 }
 
 // neighbour (d, s) of the cell ijk; -1 outside a non-periodic direction
@@ -72,17 +72,35 @@ __host__ __device__ inline long long s_nb(const SGeom& g, const int* ijk, int d,
     return j;
 }
 
-// y = A x for the structured stencil at cell i
-__device__ inline double s_apply_row(const SGeom& g, const double* __restrict__ st, const double* __restrict__ x,
-                                     long long i) {
+// couplings of cell i and its neighbours' indices (a zero coupling: the cell itself); all loads are
+// issued before the first is used -- reading coupling and value one after the other made a
+// sweep of 24^3 cells take 7.5 us
+__device__ __forceinline__ void s_row(const SGeom& g, const double* __restrict__ st, long long i, double* c, long long* nb) {
+#pragma unroll
+    for (int q = 0; q < NS; ++q) c[q] = st[q * g.N + i];
     int ijk[3];
     s_ijk(g, i, ijk);
-    double acc = st[i] * x[i];
+#pragma unroll
     for (int d = 0; d < 3; ++d)
+#pragma unroll
         for (int s = 0; s < 2; ++s) {
-            const double c = st[(1 + 2 * d + s) * g.N + i];
-            if (c != 0.0) acc += c * x[s_nb(g, ijk, d, s)];
+            const bool wrap = s ? ijk[d] + 1 >= g.n[d] : ijk[d] == 0;
+            const long long step = (long long)g.stride[d] * (wrap ? g.n[d] - 1 : 1);
+            nb[2 * d + s] = c[1 + 2 * d + s] != 0.0 ? i + ((s != 0) != wrap ? step : -step) : i;
         }
+}
+
+// (A v)_i for values v(j)
+template <class V>
+__device__ __forceinline__ double s_apply(const double* c, const long long* nb, long long i, V&& v) {
+    double x[NS];
+    x[0] = v(i);
+#pragma unroll
+    for (int q = 0; q < 6; ++q) x[1 + q] = v(nb[q]);
+    double acc = c[0] * x[0];
+#pragma unroll
+    for (int q = 0; q < 6; ++q)
+        if (c[1 + q] != 0.0) acc += c[1 + q] * x[1 + q];
     return acc;
 }
 
@@ -262,33 +280,41 @@ __global__ void k_dense_inverse(int N, const double* __restrict__ M, double* __r
     }
 }
 
-// ---- V-cycle kernels: p-levels (m modes per cell, pattern rowptr / colidx)
+// ---- V-cycle kernels: p-levels (m modes per cell, pattern rowptr / colidx). M: m as a constant for the
+// degrees in use, so that a block row's loads are all in flight (0: any m)
 // out = Dinv in (add: out += Dinv in); one thread per scalar row
-__global__ void k_bdiag(long long J, int m, const double* __restrict__ inv, const double* __restrict__ in,
+template <int M>
+__global__ void k_bdiag(unsigned n, int mr, const double* __restrict__ inv, const double* __restrict__ in,
                         double* __restrict__ out, int add) {
-    GRID_STRIDE(t, J * m) {
-        const long long j = t / m;
-        const int r = (int)(t - j * m);
-        const double* B = inv + j * (long long)m * m;
-        const double* v = in + j * m;
+    const int m = M ? M : mr;
+    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        const unsigned j = t / m, r = t - j * m;
+        const double* B = inv + (long long)j * m * m + r;
+        const double* v = in + (long long)j * m;
         double acc = 0.0;
-        for (int c = 0; c < m; ++c) acc += B[(long long)c * m + r] * v[c];
+#pragma unroll
+        for (int c = 0; c < m; ++c) acc += B[(long long)c * m] * v[c];
         out[t] = add ? out[t] + acc : acc;
     }
 }
 
 // rows r < mo of each cell of (b - A x) into out[j * mo + r] (mo = m: the full residual)
-__global__ void k_resid(long long J, int m, int mo, const long long* __restrict__ rowptr, const int* __restrict__ colidx,
+template <int M>
+__global__ void k_resid(unsigned n, int mr, int mo, const long long* __restrict__ rowptr, const int* __restrict__ colidx,
                         const double* __restrict__ vals, const double* __restrict__ x, const double* __restrict__ b,
                         double* __restrict__ out) {
-    GRID_STRIDE(t, J * mo) {
-        const long long j = t / mo;
-        const int r = (int)(t - j * mo);
-        double acc = b[j * m + r];
-        for (long long bb = rowptr[j]; bb < rowptr[j + 1]; ++bb) {
-            const double* blk = vals + bb * (long long)m * m;
+    const int m = M ? M : mr;
+    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        const unsigned j = t / mo, r = t - j * mo;
+        double acc = b[(long long)j * m + r];
+        const long long b0 = rowptr[j], b1 = rowptr[j + 1];
+        for (long long bb = b0; bb < b1; ++bb) {
+            const double* blk = vals + bb * (long long)m * m + r;
             const double* xb = x + (long long)colidx[bb] * m;
-            for (int c = 0; c < m; ++c) acc -= blk[(long long)c * m + r] * xb[c];
+            double s = 0.0;
+#pragma unroll
+            for (int c = 0; c < m; ++c) s += blk[(long long)c * m] * xb[c];
+            acc -= s;
         }
         out[t] = acc;
     }
@@ -305,64 +331,119 @@ __global__ void k_inject_add(long long J, int m, int mc, const double* __restric
 
 // ---- structured levels
 // first sweep from x = 0: x = omega b / diag
+__device__ __forceinline__ double jac_first(double b, double d) { return (d != 0.0) ? OMEGA * b / d : 0.0; }
 __global__ void k_jac0(SGeom g, const double* __restrict__ st, const double* __restrict__ b, double* __restrict__ x) {
-    GRID_STRIDE(i, g.N) {
-        const double d = st[i];
-        x[i] = (d != 0.0) ? OMEGA * b[i] / d : 0.0;
-    }
+    GRID_STRIDE(i, g.N) x[i] = jac_first(b[i], st[i]);
 }
 
 // xo = x + omega (b - A x) / diag
 __global__ void k_jac(SGeom g, const double* __restrict__ st, const double* __restrict__ b,
                       const double* __restrict__ x, double* __restrict__ xo) {
     GRID_STRIDE(i, g.N) {
-        const double d = st[i];
-        xo[i] = x[i] + ((d != 0.0) ? OMEGA * (b[i] - s_apply_row(g, st, x, i)) / d : 0.0);
+        double c[NS];
+        long long nb[6];
+        s_row(g, st, i, c, nb);
+        const double ax = s_apply(c, nb, i, [&](long long j) { return x[j]; });
+        xo[i] = x[i] + ((c[0] != 0.0) ? OMEGA * (b[i] - ax) / c[0] : 0.0);
     }
 }
 
-// bc[I] = sum over the cells of aggregate I of (b - A x)
+// the first two sweeps from x = 0 in one launch: the first sweep's values are recomputed at the neighbours
+__global__ void k_jac01(SGeom g, const double* __restrict__ st, const double* __restrict__ b, double* __restrict__ xo) {
+    GRID_STRIDE(i, g.N) {
+        double c[NS];
+        long long nb[6];
+        s_row(g, st, i, c, nb);
+        const double ax = s_apply(c, nb, i, [&](long long j) { return jac_first(b[j], st[j]); });
+        xo[i] = jac_first(b[i], c[0]) + ((c[0] != 0.0) ? OMEGA * (b[i] - ax) / c[0] : 0.0);
+    }
+}
+
+// prolongation and the sweep after it in one launch: x_j + xc[aggregate of j] at the cell and its neighbours
+__global__ void k_prolong_jac(SGeom g, SGeom gc, const double* __restrict__ st, const double* __restrict__ b,
+                              const double* __restrict__ x, const double* __restrict__ xc, double* __restrict__ xo) {
+    GRID_STRIDE(i, g.N) {
+        double c[NS];
+        long long nb[6];
+        s_row(g, st, i, c, nb);
+        auto v = [&](long long j) {
+            int jjk[3];
+            s_ijk(g, j, jjk);
+            return x[j] + xc[s_agg(gc, jjk)];
+        };
+        const double ax = s_apply(c, nb, i, v);
+        xo[i] = v(i) + ((c[0] != 0.0) ? OMEGA * (b[i] - ax) / c[0] : 0.0);
+    }
+}
+
+// bc[I] = sum over the cells of aggregate I of (b - A x): eight lanes per aggregate, one cell each (one
+// thread per aggregate walked 8 cells x 7 couplings in 27 us at 12^3 aggregates). Whole warps: the
+// launch holds 8 N threads rounded up
 __global__ void k_agg_restrict(SGeom gf, SGeom gc, const double* __restrict__ st, const double* __restrict__ b,
                                const double* __restrict__ x, double* __restrict__ bc) {
-    GRID_STRIDE(I, gc.N) {
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x, I = t >> 3;
+    const int a = (int)(t & 7);
+    double r = 0.0;
+    if (I < gc.N) {
         int IJK[3];
         s_ijk(gc, I, IJK);
-        double acc = 0.0;
-        for (int a = 0; a < 8; ++a) {
-            int ijk[3];
-            bool ok = true;
-            for (int d = 0; d < 3; ++d) {
-                ijk[d] = 2 * IJK[d] + ((a >> d) & 1);
-                ok = ok && ijk[d] < gf.n[d];
-            }
-            if (!ok) continue;
-            long long i = 0;
-            for (int d = 0; d < 3; ++d) i += (long long)ijk[d] * gf.stride[d];
-            acc += b[i] - s_apply_row(gf, st, x, i);
+        long long i = 0;
+        bool ok = true;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const int k = 2 * IJK[d] + ((a >> d) & 1);
+            ok = ok && k < gf.n[d];
+            i += (long long)k * gf.stride[d];
         }
-        bc[I] = acc;
+        if (ok) {
+            double c[NS];
+            long long nb[6];
+            s_row(gf, st, i, c, nb);
+            r = b[i] - s_apply(c, nb, i, [&](long long j) { return x[j]; });
+        }
     }
+    r += __shfl_down_sync(0xffffffffu, r, 4, 8);
+    r += __shfl_down_sync(0xffffffffu, r, 2, 8);
+    r += __shfl_down_sync(0xffffffffu, r, 1, 8);
+    if (a == 0 && I < gc.N) bc[I] = r;
 }
 
-// x[i] += xc[aggregate of i]
-__global__ void k_agg_prolong(SGeom gf, SGeom gc, const double* __restrict__ xc, double* __restrict__ x) {
-    GRID_STRIDE(i, gf.N) {
-        int ijk[3];
-        s_ijk(gf, i, ijk);
-        x[i] += xc[s_agg(gc, ijk)];
-    }
-}
-
-// x = M b, dense column-major (coarsest level)
-__global__ void k_dense_apply(long long N, const double* __restrict__ M, const double* __restrict__ b, double* __restrict__ x) {
-    GRID_STRIDE(i, N) {
-        double acc = 0.0;
-        for (long long j = 0; j < N; ++j) acc += M[j * N + i] * b[j];
-        x[i] = acc;
-    }
+// x = M b, dense column-major (coarsest level), one warp per row
+__global__ void k_dense_apply(int N, const double* __restrict__ M, const double* __restrict__ b, double* __restrict__ x) {
+    const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (i >= N) return;
+    double acc = 0.0;
+    for (int j = lane; j < N; j += 32) acc += M[(long long)j * N + i] * b[j];
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if (lane == 0) x[i] = acc;
 }
 
 int launch_grid(long long n) { return (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, 148LL * 16)); }
+
+// the number of scalar rows of a p-level fits 32 bits (J <= 2e9 cells would need 8 m TB of blocks)
+void launch_bdiag(long long J, int m, const double* inv, const double* in, double* out, int add, cudaStream_t s) {
+    const unsigned n = (unsigned)(J * m);
+    const int gr = launch_grid(J * m);
+    switch (m) {
+#define BOSSS_M(M) \
+    case M: k_bdiag<M><<<gr, 256, 0, s>>>(n, m, inv, in, out, add); break;
+        BOSSS_M(3) BOSSS_M(4) BOSSS_M(6) BOSSS_M(10) BOSSS_M(15) BOSSS_M(20)
+#undef BOSSS_M
+        default: k_bdiag<0><<<gr, 256, 0, s>>>(n, m, inv, in, out, add);
+    }
+}
+void launch_resid(long long J, int m, int mo, const long long* rowptr, const int* colidx, const double* vals, const double* x,
+                  const double* b, double* out, cudaStream_t s) {
+    const unsigned n = (unsigned)(J * mo);
+    const int gr = launch_grid(J * mo);
+    switch (m) {
+#define BOSSS_M(M) \
+    case M: k_resid<M><<<gr, 256, 0, s>>>(n, m, mo, rowptr, colidx, vals, x, b, out); break;
+        BOSSS_M(3) BOSSS_M(4) BOSSS_M(6) BOSSS_M(10) BOSSS_M(15) BOSSS_M(20)
+#undef BOSSS_M
+        default: k_resid<0><<<gr, 256, 0, s>>>(n, m, mo, rowptr, colidx, vals, x, b, out);
+    }
+}
 
 }  // namespace
 
@@ -414,7 +495,7 @@ struct bosss_pmg {
         const int gr = launch_grid(L.g.N);
         if (l + 1 == H.size()) {
             if (dense) {
-                k_dense_apply<<<gr, 256, 0, s>>>(L.g.N, dense, L.b, L.x);
+                k_dense_apply<<<(int)((L.g.N + 7) / 8), 256, 0, s>>>((int)L.g.N, dense, L.b, L.x);
             } else {
                 k_jac0<<<gr, 256, 0, s>>>(L.g, L.st, L.b, L.x);
                 for (int i = 1; i < COARSE_SWEEPS; ++i) {
@@ -425,35 +506,28 @@ struct bosss_pmg {
             return;
         }
         HLevel& C = H[l + 1];
-        k_jac0<<<gr, 256, 0, s>>>(L.g, L.st, L.b, L.x);
-        for (int i = 1; i < NU_H; ++i) {
-            k_jac<<<gr, 256, 0, s>>>(L.g, L.st, L.b, L.x, L.x2);
-            std::swap(L.x, L.x2);
-        }
-        k_agg_restrict<<<launch_grid(C.g.N), 256, 0, s>>>(L.g, C.g, L.st, L.b, L.x, C.b);
+        static_assert(NU_H == 2, "two sweeps before and after the coarse correction");
+        k_jac01<<<gr, 256, 0, s>>>(L.g, L.st, L.b, L.x);
+        k_agg_restrict<<<(unsigned)((C.g.N * 8 + 255) / 256), 256, 0, s>>>(L.g, C.g, L.st, L.b, L.x, C.b);
         cycle_h(l + 1, s);
-        k_agg_prolong<<<gr, 256, 0, s>>>(L.g, C.g, C.x, L.x);
-        for (int i = 0; i < NU_H; ++i) {
-            k_jac<<<gr, 256, 0, s>>>(L.g, L.st, L.b, L.x, L.x2);
-            std::swap(L.x, L.x2);
-        }
+        k_prolong_jac<<<gr, 256, 0, s>>>(L.g, C.g, L.st, L.b, L.x, C.x, L.x2);
+        k_jac<<<gr, 256, 0, s>>>(L.g, L.st, L.b, L.x2, L.x);
     }
 
     // p-level l: input P[l].b, output P[l].x
     void cycle_p(size_t l, cudaStream_t s) {
         PLevel& L = P[l];
-        const int gr = launch_grid(J * L.m);
-        k_bdiag<<<gr, 256, 0, s>>>(J, L.m, L.inv, L.b, L.x, 0);
+        launch_bdiag(J, L.m, L.inv, L.b, L.x, 0, s);
         const bool last = l + 1 == P.size();
         const int mc = last ? 1 : P[l + 1].m;
         double* bc = last ? H[0].b : P[l + 1].b;
-        k_resid<<<launch_grid(J * mc), 256, 0, s>>>(J, L.m, mc, rowptr, colidx, L.vals, L.x, L.b, bc);
+        launch_resid(J, L.m, mc, rowptr, colidx, L.vals, L.x, L.b, bc, s);
         if (last) cycle_h(0, s);
         else cycle_p(l + 1, s);
         const double* xc = last ? H[0].x : P[l + 1].x;
         k_inject_add<<<launch_grid(J * mc), 256, 0, s>>>(J, L.m, mc, xc, L.x);
-        k_resid<<<gr, 256, 0, s>>>(J, L.m, L.m, rowptr, colidx, L.vals, L.x, L.b, L.r);
-        k_bdiag<<<gr, 256, 0, s>>>(J, L.m, L.inv, L.r, L.x, 1);
+        launch_resid(J, L.m, L.m, rowptr, colidx, L.vals, L.x, L.b, L.r, s);
+        launch_bdiag(J, L.m, L.inv, L.r, L.x, 1, s);
     }
 
     void cycle(cudaStream_t s) {
@@ -536,7 +610,7 @@ int pmg_create(const bosss_handle* h, const bosss_bsr* A, bosss_pmg** out) {
         for (int d = 0; d < 3; ++d) {
             L.g.n[d] = d < g.D ? g.n[d] : 1;
             L.g.per[d] = d < g.D ? g.periodic[d] : 0;
-            L.g.stride[d] = d < g.D ? g.stride[d] : 1;
+            L.g.stride[d] = d < g.D ? (int)g.stride[d] : 1;
         }
         L.g.N = g.J;
         M->H.push_back(L);
@@ -551,7 +625,7 @@ int pmg_create(const bosss_handle* h, const bosss_bsr* A, bosss_pmg** out) {
         }
         C.g.stride[2] = 1;
         C.g.stride[1] = C.g.n[2];
-        C.g.stride[0] = (long long)C.g.n[1] * C.g.n[2];
+        C.g.stride[0] = C.g.n[1] * C.g.n[2];
         C.g.N = (long long)C.g.n[0] * C.g.n[1] * C.g.n[2];
         M->H.push_back(C);
     }

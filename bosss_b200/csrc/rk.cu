@@ -107,7 +107,11 @@ int bosss_b200_rk_steps_device(bosss_handle* h, int32_t stages, const double* a,
     if (rc) return rc;
     CUDA_TRY(cudaSetDevice(h->device));
     cudaStream_t st = stream ? (cudaStream_t)stream : h->stream;
-    if (!use_graph) {
+    // a graph costs its capture and instantiation (about 0.1 ms for four stages) once per call: it pays
+    // from GRAPH_STEPS steps on; below, the launches of a step (about 3 us each) run ahead of their
+    // kernels just as well. GRAPHNOTE
+    constexpr int GRAPH_STEPS = 16;
+    if (!use_graph || nsteps < GRAPH_STEPS) {
         for (int i = 0; i < nsteps; ++i) {
             rc = rk_step(h, T, dt, time + i * dt, U_dev, work_dev, st);
             if (rc) return rc;

@@ -84,52 +84,58 @@ __device__ __forceinline__ int cell_colour(const GridConst& g, long long j, cons
     return c;
 }
 
+__global__ void k_colours(GridConst g, Colouring cl, int* __restrict__ colour) {
+    for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < g.J; j += (long long)gridDim.x * blockDim.x)
+        colour[j] = cell_colour(g, j, cl);
+}
+
 // probe: V[j*Nd + i] = 1 for cells of colour `col` and local column `i0`, else 0
-__global__ void k_probe(GridConst g, Colouring cl, int col, int Nd, int i0, double* V) {
-    const long long n = (long long)g.J * Nd;
+__global__ void k_probe(long long n, const int* __restrict__ colour, int col, int Nd, int i0, double* V) {
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const long long j = t / Nd;
-        const int i = (int)(t - j * Nd);
-        V[t] = (i == i0 && cell_colour(g, j, cl) == col) ? 1.0 : 0.0;
+        const unsigned j = n < 4000000000LL ? (unsigned)t / (unsigned)Nd : (unsigned)(t / Nd);
+        const int i = (int)(t - (long long)j * Nd);
+        V[t] = (i == i0 && colour[j] == col) ? 1.0 : 0.0;
     }
 }
 
 // scatter JV into column i0 of every block whose column cell has colour `col`
 // (blocks column-major: vals[b*br*bc + i0*br + r])
-__global__ void k_scatter(GridConst g, Colouring cl, int col, int i0, int br, int bc,
+__global__ void k_scatter(long long nrows, const int* __restrict__ colour, int col, int i0, int br, int bc,
                           const long long* __restrict__ rowptr, const int* __restrict__ colidx,
                           const double* __restrict__ JV, double* __restrict__ vals) {
-    const long long nrows = (long long)g.J * br;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < nrows; t += (long long)gridDim.x * blockDim.x) {
-        const long long j = t / br;
-        const int r = (int)(t - j * br);
-        for (long long b = rowptr[j]; b < rowptr[j + 1]; ++b)
-            if (cell_colour(g, colidx[b], cl) == col) vals[b * (long long)br * bc + (long long)i0 * br + r] = JV[t];
+        const unsigned j = nrows < 4000000000LL ? (unsigned)t / (unsigned)br : (unsigned)(t / br);
+        const int r = (int)(t - (long long)j * br);
+        const long long b0 = rowptr[j], b1 = rowptr[j + 1];
+        for (long long b = b0; b < b1; ++b)
+            if (colour[colidx[b]] == col) vals[b * (long long)br * bc + (long long)i0 * br + r] = JV[t];
     }
 }
 
 // cell-block pattern: self first, then the face neighbours (duplicates dropped)
 static void block_pattern(const GridConst& g, std::vector<int64_t>& rowptr, std::vector<int32_t>& colidx) {
-    rowptr.assign(1, 0);
-    colidx.clear();
+    rowptr.resize((size_t)g.J + 1);
+    colidx.resize((size_t)g.J * (2 * g.D + 1));
+    rowptr[0] = 0;
+    size_t n = 0;
     for (long long j = 0; j < g.J; ++j) {
-        int ijk[3] = {0, 0, 0};
-        for (int d = 0; d < g.D; ++d) ijk[d] = (int)((j / g.stride[d]) % g.n[d]);
-        std::vector<int32_t> cols{(int32_t)j};
-        for (int d = 0; d < g.D; ++d)
+        const size_t first = n;
+        colidx[n++] = (int32_t)j;
+        for (int d = 0; d < g.D; ++d) {
+            const int nd = g.n[d], i = (int)(((unsigned)j / (unsigned)g.stride[d]) % (unsigned)nd);
             for (int s = 0; s < 2; ++s) {
-                int i = ijk[d] + (s ? 1 : -1);
-                if (i < 0 || i >= g.n[d]) {
-                    if (!g.periodic[d]) continue;
-                    i = (i + g.n[d]) % g.n[d];
-                }
-                long long nb = 0;
-                for (int dd = 0; dd < g.D; ++dd) nb += (long long)((dd == d) ? i : ijk[dd]) * g.stride[dd];
-                if (std::find(cols.begin(), cols.end(), (int32_t)nb) == cols.end()) cols.push_back((int32_t)nb);
+                const bool wrap = s ? i + 1 >= nd : i == 0;
+                if (wrap && !g.periodic[d]) continue;
+                const long long step = (wrap ? nd - 1 : 1) * g.stride[d];
+                const int32_t nb = (int32_t)((s != 0) != wrap ? j + step : j - step);
+                bool seen = false;
+                for (size_t k = first; k < n; ++k) seen = seen || colidx[k] == nb;
+                if (!seen) colidx[n++] = nb;
             }
-        colidx.insert(colidx.end(), cols.begin(), cols.end());
-        rowptr.push_back((int64_t)colidx.size());
+        }
+        rowptr[(size_t)j + 1] = (int64_t)n;
     }
+    colidx.resize(n);
 }
 
 static int grid_of(long long n) { return (int)std::min<long long>((n + 255) / 256, 148LL * 16); }
@@ -204,31 +210,37 @@ static int assemble(bosss_handle* h, const double* U_dev, double time, bosss_bsr
     if (e == cudaSuccess) e = cudaMemcpy(A->d_colidx, ci.data(), sizeof(int32_t) * ci.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemsetAsync(A->d_vals, 0, sizeof(double) * bs * ci.size(), s);
     double *V = nullptr, *JV = nullptr;
+    int* colour = nullptr;   // of every cell: found once, read by all probes and scatters
     if (e == cudaSuccess) e = cudaMalloc(&V, sizeof(double) * h->ndom);
     if (e == cudaSuccess) e = cudaMalloc(&JV, sizeof(double) * h->ncod);
+    if (e == cudaSuccess) e = cudaMalloc(&colour, sizeof(int) * std::max<int64_t>(g.J, 1));
     if (e != cudaSuccess) {
         cudaFree(V);
         cudaFree(JV);
+        cudaFree(colour);
         return bail(e);
     }
     const Colouring c = make_colouring(g);
+    k_colours<<<grid_of(g.J), 256, 0, s>>>(g, c, colour);
     for (int col = 0; col < c.ncol && e == cudaSuccess; ++col)
         for (int i0 = 0; i0 < Nd && e == cudaSuccess; ++i0) {
-            k_probe<<<grid_of(h->ndom), 256, 0, s>>>(g, c, col, Nd, i0, V);
+            k_probe<<<grid_of(h->ndom), 256, 0, s>>>(h->ndom, colour, col, Nd, i0, V);
             int rc = run_mode(h, MODE_JVP, 1.0, 0.0, U_dev, V, JV, time, s);
             if (rc) {
                 cudaFree(V);
                 cudaFree(JV);
+                cudaFree(colour);
                 bosss_b200_bsr_destroy(A);
                 return rc;
             }
-            k_scatter<<<grid_of(h->ncod), 256, 0, s>>>(g, c, col, i0, Nc, Nd,
-                                                       (const long long*)A->d_rowptr, A->d_colidx, JV, A->d_vals);
+            k_scatter<<<grid_of(h->ncod), 256, 0, s>>>(h->ncod, colour, col, i0, Nc, Nd, (const long long*)A->d_rowptr,
+                                                       A->d_colidx, JV, A->d_vals);
             e = cudaGetLastError();
         }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     cudaFree(V);
     cudaFree(JV);
+    cudaFree(colour);
     if (e != cudaSuccess) return bail(e);
     *out = A;
     return BOSSS_OK;
@@ -710,9 +722,10 @@ int bosss_b200_batch_solve(bosss_batch* B, int32_t transpose, const double* dt, 
     bosss_pmg* mg = nullptr;
     float *r32 = nullptr, *c32 = nullptr, *t32 = nullptr, *inv = nullptr;
     long long* rp = nullptr;
-    int* sing = nullptr;
+    int *sing = nullptr, *colour = nullptr;
     KrylovWork<float> kw;
     auto cleanup = [&]() {
+        cudaFree(colour);
         cudaFree(r64);
         cudaFree(t64);
         cudaFree(y64);
@@ -740,6 +753,7 @@ int bosss_b200_batch_solve(bosss_batch* B, int32_t transpose, const double* dt, 
     if (e == cudaSuccess && o.precond == 1) e = cudaMalloc(&blk, sizeof(double) * bmax);
     if (e == cudaSuccess && o.precond == 1) e = cudaMalloc(&inv, sizeof(float) * bmax);
     if (e == cudaSuccess && o.precond == 1) e = cudaMalloc(&rp, sizeof(long long) * (nmax + 1));
+    if (e == cudaSuccess && o.precond == 1) e = cudaMalloc(&colour, sizeof(int) * nmax);
     if (e == cudaSuccess) e = cudaMalloc(&sing, sizeof(int));
     if (e == cudaSuccess) e = kw.alloc(nmax, o.restart);
     if (e == cudaSuccess && u0) e = cudaMemsetAsync(u0, 0, sizeof(double) * nmax, s);
@@ -775,9 +789,10 @@ int bosss_b200_batch_solve(bosss_batch* B, int32_t transpose, const double* dt, 
         // block-Jacobi: the diagonal cell blocks of I/dt + J, probed over a distance-1 colouring
         if (o.precond == 1) {
             const Colouring c = make_colouring1(g);
+            k_colours<<<grid_of(g.J), 256, 0, s>>>(g, c, colour);
             for (int col = 0; col < c.ncol && !rc; ++col)
                 for (int i0 = 0; i0 < nb && !rc; ++i0) {
-                    k_probe<<<grid_of(n), 256, 0, s>>>(g, c, col, nb, i0, t64);
+                    k_probe<<<grid_of(n), 256, 0, s>>>(n, colour, col, nb, i0, t64);
                     rc = run_mode(h, MODE_JVP, 1.0, 0.0, U, t64, y64, 0.0, s);
                     if (!rc)
                         k_scatter_diag<<<grid_of(n), 256, 0, s>>>(g, c, col, nb, i0, idt, y64, blk);

@@ -471,150 +471,252 @@ __device__ __forceinline__ double bgrad(const double (&L)[3][K + 1], const doubl
     return L[0][a] * L[1][b] * dL[2][c];
 }
 
+// sums of N values over the 32 lanes of a warp, value i of the result in lane `i % 32` (N <= 32): each
+// step exchanges half of the values with the partner lane, 31 exchanges instead of 5 N. The order of
+// the additions is fixed, so the result is the same bits run to run.
+template <int N>
+__device__ __forceinline__ double warp_sums(double (&v)[32]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+            // a lane with bit o keeps the values i + o, the other one the values i
+            const bool lo = i < N, hi = i + o < N;
+            if (!lo && !hi) continue;
+            const double send = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    return v[0];
+}
+
+// Contributions of one cut item, one warp per item, the nodes over its lanes.
+//  volume: u and grad u at the node from the coefficients, the volume form, 4 sums per node tested
+//          with the modes: NP sums over the warp;
+//  face:   the forms read the normal derivative only, so the coefficients are first contracted with
+//          the traces along the normal (NPAIR values and normal derivatives per side, once per
+//          item); a node then costs 4 NPAIR instead of 8 NP products, and 3 NPAIR sums (g, G of
+//          both sides on the face modes) go over the warp before they are expanded to the modes.
+// The item's contributions go to its slot of item_out (own cell, then the face neighbour), which
+// k_cut_gather adds into the cells in a fixed order -- no atomics, so the result is the same bits
+// run to run. Latency-bound: items have 8 to 125 nodes; the first version (64 threads per item,
+// full gradients, 2 NP block reductions of 5 steps) took 115 us per species at 80^3, k = 2.
 template <int K>
-__global__ void k_cut_eval(const CutItem* __restrict__ items, int nitems, const double* __restrict__ nodes,
-                           const double* __restrict__ weights, EvalArgs a, double* __restrict__ item_out) {
-    using Phys = PhysScalar<3, true>;
-    constexpr int NP = np_of(3, K);
-    const int r = blockIdx.x;
-    if (r >= nitems) return;
+__global__ void __launch_bounds__(128) k_cut_eval(const CutItem* __restrict__ items, int nitems, const double* __restrict__ nodes,
+                                                  const double* __restrict__ weights, EvalArgs a, double* __restrict__ item_out) {
+    constexpr int NP = np_of(3, K), NPAIR = (K + 1) * (K + 2) / 2;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int r = blockIdx.x * 4 + warp;
+    __shared__ double buf[4][2 * NP + 4 * NPAIR];
+    if (r >= nitems) return;   // whole warps; the kernel has no block barrier
+    double* cA = buf[warp];
+    double* cB = cA + NP;
+    double* tr = cB + NP;      // face: u_A, du_A, u_B, du_B on the face modes
     const CutItem it = items[r];
     const GridConst& g = a.g;
-    __shared__ double cA[NP], cB[NP];
+    const PhysParams& ph = a.ph;
     int ijk[3];
     cell_ijk(g, it.cell, ijk);
     long long other = -1;
     if (it.dim == 2) other = neighbour(g, ijk, it.dir, it.side);
-    for (int n = threadIdx.x; n < NP; n += blockDim.x) {
+    for (int n = lane; n < NP; n += 32) {
         cA[n] = a.U[it.cell * NP + n];
         cB[n] = (other >= 0) ? a.U[other * NP + n] : 0.0;
     }
-    __syncthreads();
-    double rA[NP], rB[NP];
-    for (int n = 0; n < NP; ++n) rA[n] = rB[n] = 0.0;
+    __syncwarp();
     const double sc = g.scaling;
-    for (int j = threadIdx.x; j < it.nnodes; j += blockDim.x) {
-        const double* t = nodes + (it.node_off + j) * 3;
-        const double wq = weights[it.node_off + j];
-        // reference coordinates of the node in the own cell (and the neighbour)
-        double xiA[3], xiB[3];
-        if (it.dim == 3) {
-            xiA[0] = t[0];
-            xiA[1] = t[1];
-            xiA[2] = t[2];
-        } else {
-            const int t1 = (it.dir == 0) ? 1 : 0, t2 = (it.dir == 2) ? 1 : 2;
-            xiA[it.dir] = it.side ? 1.0 : -1.0;
-            xiA[t1] = t[0];
-            xiA[t2] = t[1];
-            xiB[it.dir] = -xiA[it.dir];
-            xiB[t1] = t[0];
-            xiB[t2] = t[1];
-        }
-        double LA[3][K + 1], dLA[3][K + 1], LB[3][K + 1], dLB[3][K + 1];
-        for (int d = 0; d < 3; ++d) {
-            legendre_vals(K, xiA[d], LA[d], dLA[d]);
-            if (it.dim == 2) legendre_vals(K, xiB[d], LB[d], dLB[d]);
-        }
-        double uA = 0.0, GA[1][3] = {{0.0, 0.0, 0.0}};
+    const bool tran = ph.has_transport != 0, sip = ph.has_sip != 0;
+    const double nu0 = sip ? ph.nu0 : 0.0, nu2 = sip ? ph.nu2 : 0.0;
+    double* o0 = item_out + ((long long)r * 2) * NP;
+    if (it.dim == 3) {
+        double acc[NP];
 #pragma unroll
-        #pragma unroll
-        for (int n = 0; n < NP; ++n) {
-            uA += cA[n] * bphi<K>(LA, n);
-            for (int d = 0; d < 3; ++d) GA[0][d] += cA[n] * bgrad<K>(LA, dLA, n, d);
-        }
-        uA *= sc;
-        for (int d = 0; d < 3; ++d) GA[0][d] *= sc * g.twoh[d];
-        double x[3];
-        for (int d = 0; d < 3; ++d) x[d] = g.lo[d] + (ijk[d] + 0.5 + 0.5 * xiA[d]) * g.h[d];
-        if (it.dim == 3) {
-            double U1[1] = {uA}, fV[1] = {0.0}, fG[1][3] = {{0.0, 0.0, 0.0}};
-            Phys::volume(a.ph, U1, GA, x, fV, fG);
-            const double fac = wq * g.detJ * sc;
-            #pragma unroll
+        for (int n = 0; n < NP; ++n) acc[n] = 0.0;
+        for (int j = lane; j < it.nnodes; j += 32) {
+            const double* t = nodes + (it.node_off + j) * 3;
+            const double fac = weights[it.node_off + j] * g.detJ * sc;
+            double L[3][K + 1], dL[3][K + 1];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) legendre_vals(K, t[d], L[d], dL[d]);
+            double u = 0.0, G[3] = {0.0, 0.0, 0.0};
+#pragma unroll
             for (int n = 0; n < NP; ++n) {
-                double acc = fV[0] * bphi<K>(LA, n);
-                for (int d = 0; d < 3; ++d) acc += fG[0][d] * bgrad<K>(LA, dLA, n, d) * g.twoh[d];
-                rA[n] += fac * acc;
+                int p, q, s;
+                mode3<K>(n, p, q, s);
+                const double c = cA[n], yz = L[1][q] * L[2][s];
+                u += c * (L[0][p] * yz);
+                G[0] += c * (dL[0][p] * yz);
+                G[1] += c * (L[0][p] * dL[1][q] * L[2][s]);
+                G[2] += c * (L[0][p] * L[1][q] * dL[2][s]);
             }
+            u *= sc;
+            const double nu = fma(nu2 * u, u, nu0);
+            double f[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                f[d] = -(nu * (G[d] * (sc * g.twoh[d])) + (tran ? ph.vel[d] * u : 0.0)) * (fac * g.twoh[d]);
+            const double fv = ph.has_source ? ph.src * fac : 0.0;
+#pragma unroll
+            for (int n = 0; n < NP; ++n) {
+                int p, q, s;
+                mode3<K>(n, p, q, s);
+                const double yz = L[1][q] * L[2][s];
+                acc[n] += L[0][p] * (fv * yz + f[1] * (dL[1][q] * L[2][s]) + f[2] * (L[1][q] * dL[2][s])) + f[0] * (dL[0][p] * yz);
+            }
+        }
+#pragma unroll
+        for (int n0 = 0; n0 < NP; n0 += 32) {
+            double v[32];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = n0 + i < NP ? acc[n0 + i] : 0.0;
+            const double s = warp_sums<32>(v);
+            const int n = n0 + lane;
+            if (n < NP) {
+                o0[n] = a.alpha * s;
+                o0[NP + n] = 0.0;
+            }
+        }
+        return;
+    }
+    // ---- face: traces along the normal
+    const int dir = it.dir;
+    const double nA = it.side ? 1.0 : -1.0;   // the own cell's side of the face
+    const int t1 = (dir == 0) ? 1 : 0, t2 = (dir == 2) ? 1 : 2;
+    double LA[K + 1], dLA[K + 1], LB[K + 1], dLB[K + 1];
+    legendre_vals(K, nA, LA, dLA);
+    legendre_vals(K, -nA, LB, dLB);
+    for (int i = lane; i < NPAIR; i += 32) {
+        int p = 0, q = i;
+        while (q > K - p) {
+            q -= K + 1 - p;
+            ++p;
+        }
+        double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int m = 0; m <= K; ++m)
+            if (m <= K - p - q) {
+                const int n = dir == 0 ? bosss::mode3(m, p, q) : dir == 1 ? bosss::mode3(p, m, q) : bosss::mode3(p, q, m);
+                s[0] += cA[n] * LA[m];
+                s[1] += cA[n] * dLA[m];
+                s[2] += cB[n] * LB[m];
+                s[3] += cB[n] * dLB[m];
+            }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) tr[k * NPAIR + i] = s[k] * ((k & 1) ? sc * g.twoh[dir] : sc);
+    }
+    __syncwarp();
+    const bool selfLower = it.side == 1;      // reference roles: IN = lower cell, normal +e_dir
+    double pen;
+    if (other >= 0) {
+        int ijk2[3] = {ijk[0], ijk[1], ijk[2]};
+        ijk2[dir] = (int)((other / g.stride[dir]) % g.n[dir]);
+        pen = ph.pen * fmax(penalty_size(a.cell_pf, g, ijk), penalty_size(a.cell_pf, g, ijk2));
+    } else {
+        pen = 2.0 * ph.pen * penalty_size(a.cell_pf, g, ijk);
+    }
+    const double vel = tran ? ph.vel[dir] : 0.0;
+    double w[3][NPAIR];   // g of the own cell, G of the own cell and of the neighbour on the face modes
+#pragma unroll
+    for (int i = 0; i < NPAIR; ++i) w[0][i] = w[1][i] = w[2][i] = 0.0;
+    for (int j = lane; j < it.nnodes; j += 32) {
+        const double* t = nodes + (it.node_off + j) * 3;
+        const double fac = weights[it.node_off + j] * g.faceSG[dir] * sc;
+        double L1[K + 1], L2[K + 1], d1[K + 1], d2[K + 1], f[NPAIR];
+        legendre_vals(K, t[0], L1, d1);
+        legendre_vals(K, t[1], L2, d2);
+        double v[4] = {0.0, 0.0, 0.0, 0.0};
+        int i = 0;
+#pragma unroll
+        for (int p = 0; p <= K; ++p)
+#pragma unroll
+            for (int q = 0; q <= K - p; ++q, ++i) {
+                f[i] = L1[p] * L2[q];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) v[k] += tr[k * NPAIR + i] * f[i];
+            }
+        double gs, GA, GB;
+        if (other >= 0) {
+            const double uI = selfLower ? v[0] : v[2], dI = selfLower ? v[1] : v[3];
+            const double uO = selfLower ? v[2] : v[0], dO = selfLower ? v[3] : v[1];
+            const double nI = fma(nu2 * uI, uI, nu0), nO = fma(nu2 * uO, uO, nu0), J = uI - uO;
+            const double nM = fabs(nI) > fabs(nO) ? nI : nO;
+            const double gi = 0.5 * (nI * dI + nO * dO) - pen * nM * J + vel * (vel > 0.0 ? uI : uO);
+            gs = selfLower ? gi : -gi;
+            GA = 0.5 * (selfLower ? nI : nO) * J;
+            GB = 0.5 * (selfLower ? nO : nI) * J;
         } else {
-            const double fac = wq * g.faceSG[it.dir] * sc;
-            double nrm[3] = {0.0, 0.0, 0.0};
-            if (other >= 0) {
-                double uB = 0.0, GB[1][3] = {{0.0, 0.0, 0.0}};
-                #pragma unroll
-                for (int n = 0; n < NP; ++n) {
-                    uB += cB[n] * bphi<K>(LB, n);
-                    for (int d = 0; d < 3; ++d) GB[0][d] += cB[n] * bgrad<K>(LB, dLB, n, d);
-                }
-                uB *= sc;
-                for (int d = 0; d < 3; ++d) GB[0][d] *= sc * g.twoh[d];
-                // reference roles: IN = lower cell, normal +e_dir
-                const bool selfLower = it.side == 1;
-                nrm[it.dir] = 1.0;
-                int ijk2[3] = {ijk[0], ijk[1], ijk[2]};
-                ijk2[it.dir] = (int)((other / g.stride[it.dir]) % g.n[it.dir]);
-                const double pnlty = a.ph.pen * fmax(penalty_size(a.cell_pf, g, ijk), penalty_size(a.cell_pf, g, ijk2));
-                double U_in[1], U_out[1], G_in[1][3], G_out[1][3];
-                U_in[0] = selfLower ? uA : uB;
-                U_out[0] = selfLower ? uB : uA;
-                for (int d = 0; d < 3; ++d) {
-                    G_in[0][d] = selfLower ? GA[0][d] : GB[0][d];
-                    G_out[0][d] = selfLower ? GB[0][d] : GA[0][d];
-                }
-                double gi[1] = {0.0}, go[1] = {0.0}, Gi[1][3] = {{0, 0, 0}}, Go[1][3] = {{0, 0, 0}};
-                Phys::inner(a.ph, pnlty, U_in, G_in, U_out, G_out, nrm, x, gi, Gi, go, Go);
-                // own cell A gets IN terms if it is the lower cell
-                const double gsA = selfLower ? gi[0] : go[0], gsB = selfLower ? go[0] : gi[0];
-                const double* GsA = selfLower ? Gi[0] : Go[0];
-                const double* GsB = selfLower ? Go[0] : Gi[0];
-                #pragma unroll
-                for (int n = 0; n < NP; ++n) {
-                    double accA = gsA * bphi<K>(LA, n), accB = gsB * bphi<K>(LB, n);
-                    for (int d = 0; d < 3; ++d) {
-                        accA += GsA[d] * bgrad<K>(LA, dLA, n, d) * g.twoh[d];
-                        accB += GsB[d] * bgrad<K>(LB, dLB, n, d) * g.twoh[d];
-                    }
-                    rA[n] += fac * accA;
-                    rB[n] += fac * accB;
-                }
-            } else {
-                nrm[it.dir] = it.side ? 1.0 : -1.0;
-                const double pnlty = 2.0 * a.ph.pen * penalty_size(a.cell_pf, g, ijk);
-                double U1[1] = {uA}, gi[1] = {0.0}, Gi[1][3] = {{0, 0, 0}};
-                Phys::boundary(a.ph, pnlty, U1, GA, nrm, x, nullptr, 0, gi, Gi);
-                #pragma unroll
-                for (int n = 0; n < NP; ++n) {
-                    double acc = gi[0] * bphi<K>(LA, n);
-                    for (int d = 0; d < 3; ++d) acc += Gi[0][d] * bgrad<K>(LA, dLA, n, d) * g.twoh[d];
-                    rA[n] += fac * acc;
-                }
+            double x[3];
+            x[dir] = g.lo[dir] + (ijk[dir] + 0.5 + 0.5 * nA) * g.h[dir];
+            x[t1] = g.lo[t1] + (ijk[t1] + 0.5 + 0.5 * t[0]) * g.h[t1];
+            x[t2] = g.lo[t2] + (ijk[t2] + 0.5 + 0.5 * t[1]) * g.h[t2];
+            const double an = vel * nA;
+            gs = an >= 0.0 ? an * v[0] : 0.0;
+            GA = GB = 0.0;
+            if (sip && ph.dirichlet) {
+                double gD = ph.g0;
+#pragma unroll
+                for (int d = 0; d < 3; ++d) gD += ph.g1[d] * x[d] + ph.g2[d] * x[d] * x[d];
+                const double nu = fma(nu2 * v[0], v[0], nu0), df = v[0] - gD;
+                gs += nu * v[1] * nA - nu * df * pen;
+                GA = nu * df * nA;
             }
         }
-    }
-    // fixed-order reduction over the block (2 warps): warp shuffles, then the two warps' sums;
-    // the item's contributions go to its slot of item_out (own cell, then the face
-    // neighbour), which k_cut_gather adds into the cells in a fixed order -- no atomics, so
-    // the result is the same bits run to run
-    __shared__ double red[2][2][NP];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    #pragma unroll
-    for (int n = 0; n < NP; ++n) {
-        double va = rA[n], vb = rB[n];
-        for (int o = 16; o > 0; o >>= 1) {
-            va += __shfl_down_sync(0xffffffffu, va, o);
-            vb += __shfl_down_sync(0xffffffffu, vb, o);
-        }
-        if (lane == 0) {
-            red[warp][0][n] = va;
-            red[warp][1][n] = vb;
+        gs *= fac;
+        GA *= fac * g.twoh[dir];
+        GB *= fac * g.twoh[dir];
+#pragma unroll
+        for (int k = 0; k < NPAIR; ++k) {
+            w[0][k] += gs * f[k];
+            w[1][k] += GA * f[k];
+            w[2][k] += GB * f[k];
         }
     }
-    __syncthreads();
-    const bool two = it.dim == 2 && other >= 0;
-    for (int n = threadIdx.x; n < NP; n += blockDim.x) {
-        item_out[((long long)r * 2 + 0) * NP + n] = a.alpha * (red[0][0][n] + red[1][0][n]);
-        item_out[((long long)r * 2 + 1) * NP + n] = two ? a.alpha * (red[0][1][n] + red[1][1][n]) : 0.0;
+    // sums over the warp, in groups of 32
+    __syncwarp();
+#pragma unroll
+    for (int n0 = 0; n0 < 3 * NPAIR; n0 += 32) {
+        double v[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = n0 + i < 3 * NPAIR ? w[(n0 + i) / NPAIR][(n0 + i) % NPAIR] : 0.0;
+        const double s = warp_sums<32>(v);
+        if (n0 + lane < 3 * NPAIR) tr[n0 + lane] = s;
+    }
+    __syncwarp();
+    const bool two = other >= 0;
+    for (int n = lane; n < NP; n += 32) {
+        // exponents of mode n
+        int p3[3] = {0, 0, 0};
+        {
+            int m = n, deg = 0;
+            while (m >= (deg + 1) * (deg + 2) / 2) {
+                m -= (deg + 1) * (deg + 2) / 2;
+                ++deg;
+            }
+            int aa = 0;
+            while (m > deg - aa) {
+                m -= deg - aa + 1;
+                ++aa;
+            }
+            p3[0] = aa;
+            p3[1] = m;
+            p3[2] = deg - aa - m;
+        }
+        const int m = dir == 0 ? p3[0] : dir == 1 ? p3[1] : p3[2];
+        const int p = dir == 0 ? p3[1] : p3[0], q = dir == 2 ? p3[1] : p3[2];
+        const int i = p * (K + 1) - p * (p - 1) / 2 + q;
+        double lA = 0.0, dA = 0.0, lB = 0.0, dB = 0.0;
+#pragma unroll
+        for (int k = 0; k <= K; ++k)
+            if (k == m) {
+                lA = LA[k];
+                dA = dLA[k];
+                lB = LB[k];
+                dB = dLB[k];
+            }
+        o0[n] = a.alpha * (tr[i] * lA + tr[NPAIR + i] * dA);
+        o0[NP + n] = two ? a.alpha * (-tr[i] * lB + tr[2 * NPAIR + i] * dB) : 0.0;
     }
 }
 
@@ -663,42 +765,36 @@ __global__ void k_interface_eval(const long long* __restrict__ cells, const long
     const int r = blockIdx.x;
     if (r >= ncells) return;
     const long long cell = cells[r];
-    __shared__ double cA[NP], cB[NP], RA[NP], RB[NP];
+    __shared__ double cA[NP], cB[NP], red[2][2 * NP];
     for (int n = threadIdx.x; n < NP; n += blockDim.x) {
         cA[n] = UA[cell * NP + n];
         cB[n] = UB[cell * NP + n];
-        RA[n] = 0.0;
-        RB[n] = 0.0;
     }
     __syncthreads();
     const double pen = f.pen * fmax(f.pfA[cell], f.pfB[cell]);
     const double sc = g.scaling;
-    double rA[NP], rB[NP];
-    for (int n = 0; n < NP; ++n) rA[n] = rB[n] = 0.0;
+    double rr[2 * NP];   // sums for species A, then B
+#pragma unroll
+    for (int n = 0; n < 2 * NP; ++n) rr[n] = 0.0;
     const long long j0 = node_off[r], j1 = node_off[r + 1];
     for (long long j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
         const double* xi = nodes + 3 * j;
-        const double* N = normals + 3 * j;
+        const double N[3] = {normals[3 * j] * g.twoh[0], normals[3 * j + 1] * g.twoh[1], normals[3 * j + 2] * g.twoh[2]};
         double L[3][K + 1], dL[3][K + 1];
+#pragma unroll
         for (int d = 0; d < 3; ++d) legendre_vals(K, xi[d], L[d], dL[d]);
         double ph[NP], gn[NP];   // basis value and normal derivative (physical, without sc)
         double uA = 0.0, uB = 0.0, gA = 0.0, gB = 0.0;
-        {
-            int nn = 0;
-            for (int deg = 0; deg <= K; ++deg)
-                for (int aa = 0; aa <= deg; ++aa)
-                    for (int bb = 0; bb <= deg - aa; ++bb) {
-                        const int cc = deg - aa - bb;
-                        ph[nn] = L[0][aa] * L[1][bb] * L[2][cc];
-                        gn[nn] = dL[0][aa] * L[1][bb] * L[2][cc] * g.twoh[0] * N[0] +
-                                 L[0][aa] * dL[1][bb] * L[2][cc] * g.twoh[1] * N[1] +
-                                 L[0][aa] * L[1][bb] * dL[2][cc] * g.twoh[2] * N[2];
-                        uA += cA[nn] * ph[nn];
-                        uB += cB[nn] * ph[nn];
-                        gA += cA[nn] * gn[nn];
-                        gB += cB[nn] * gn[nn];
-                        ++nn;
-                    }
+#pragma unroll
+        for (int n = 0; n < NP; ++n) {
+            int p, q, s;
+            mode3<K>(n, p, q, s);
+            ph[n] = L[0][p] * L[1][q] * L[2][s];
+            gn[n] = dL[0][p] * L[1][q] * L[2][s] * N[0] + L[0][p] * dL[1][q] * L[2][s] * N[1] + L[0][p] * L[1][q] * dL[2][s] * N[2];
+            uA += cA[n] * ph[n];
+            uB += cB[n] * ph[n];
+            gA += cA[n] * gn[n];
+            gB += cB[n] * gn[n];
         }
         uA *= sc;
         uB *= sc;
@@ -708,34 +804,27 @@ __global__ void k_interface_eval(const long long* __restrict__ cells, const long
         const double flux = f.muA * f.omA * gA + f.muB * f.omB * gB - pen * jump;
         const double w = weights[j] * sc;
         const double symA = f.muA * f.omA * jump, symB = f.muB * f.omB * jump;
+#pragma unroll
         for (int n = 0; n < NP; ++n) {
-            rA[n] += w * (flux * ph[n] + symA * gn[n]);
-            rB[n] += w * (-flux * ph[n] + symB * gn[n]);
+            rr[n] += w * (flux * ph[n] + symA * gn[n]);
+            rr[NP + n] += w * (-flux * ph[n] + symB * gn[n]);
         }
     }
     // fixed-order reduction over the block (2 warps of 32): the same bits run to run
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int n = 0; n < NP; ++n) {
-        double va = rA[n], vb = rB[n];
-        for (int o = 16; o > 0; o >>= 1) {
-            va += __shfl_down_sync(0xffffffffu, va, o);
-            vb += __shfl_down_sync(0xffffffffu, vb, o);
-        }
-        if (lane == 0 && warp == 1) {
-            RA[n] = va;
-            RB[n] = vb;
-        }
-        if (lane == 0 && warp == 0) {
-            rA[n] = va;
-            rB[n] = vb;
-        }
+#pragma unroll
+    for (int n0 = 0; n0 < 2 * NP; n0 += 32) {
+        double v[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = n0 + i < 2 * NP ? rr[n0 + i] : 0.0;
+        const double s = warp_sums<32>(v);
+        if (n0 + lane < 2 * NP) red[warp][n0 + lane] = s;
     }
     __syncthreads();
-    if (threadIdx.x == 0)
-        for (int n = 0; n < NP; ++n) {
-            outA[cell * NP + n] += f.alpha * (rA[n] + RA[n]);
-            outB[cell * NP + n] += f.alpha * (rB[n] + RB[n]);
-        }
+    for (int n = threadIdx.x; n < 2 * NP; n += blockDim.x) {
+        double* o = n < NP ? outA + cell * NP + n : outB + cell * NP + (n - NP);
+        *o += f.alpha * (red[0][n] + red[1][n]);
+    }
 }
 
 // Surface rule of the sphere |x - c| = R inside the box [lo, hi] (physical coordinates), by
@@ -1853,10 +1942,10 @@ int bosss_b200_xdg_evaluate_device(bosss_xdg* X, int32_t species, double alpha, 
         a.alpha = alpha;
         a.time = time;
         switch (X->K) {
-            case 1: k_cut_eval<1><<<n, 64, 0, st>>>(X->d_items[s], n, X->d_nodes[s], X->d_weights[s], a, X->d_item_out[s]); break;
-            case 2: k_cut_eval<2><<<n, 64, 0, st>>>(X->d_items[s], n, X->d_nodes[s], X->d_weights[s], a, X->d_item_out[s]); break;
-            case 3: k_cut_eval<3><<<n, 64, 0, st>>>(X->d_items[s], n, X->d_nodes[s], X->d_weights[s], a, X->d_item_out[s]); break;
-            default: k_cut_eval<4><<<n, 64, 0, st>>>(X->d_items[s], n, X->d_nodes[s], X->d_weights[s], a, X->d_item_out[s]); break;
+            case 1: k_cut_eval<1><<<(n + 3) / 4, 128, 0, st>>>(X->d_items[s], n, X->d_nodes[s], X->d_weights[s], a, X->d_item_out[s]); break;
+            case 2: k_cut_eval<2><<<(n + 3) / 4, 128, 0, st>>>(X->d_items[s], n, X->d_nodes[s], X->d_weights[s], a, X->d_item_out[s]); break;
+            case 3: k_cut_eval<3><<<(n + 3) / 4, 128, 0, st>>>(X->d_items[s], n, X->d_nodes[s], X->d_weights[s], a, X->d_item_out[s]); break;
+            default: k_cut_eval<4><<<(n + 3) / 4, 128, 0, st>>>(X->d_items[s], n, X->d_nodes[s], X->d_weights[s], a, X->d_item_out[s]); break;
         }
         CUDA_TRY(cudaGetLastError());
         const long long nc = X->n_gcells[s], NPc = np_of(3, X->K);
