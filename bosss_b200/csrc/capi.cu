@@ -806,7 +806,9 @@ int bosss_b200_apply_device(bosss_handle* h, int32_t mode, double alpha, double 
 // when that direction is periodic), and each chunk's outputs stream out on a second copy stream
 // while later chunks are still computing. Small problems, and the opt-in NaN check, run as one
 // chunk. Returns after the last output has reached the host. A chunk's residual and VJP run on two
-// streams: each alone fills the chip for a fraction of a wave only. CHUNKNOTE
+// streams: each alone fills the chip for a fraction of a wave only (Euler 32^3 k=3, 1.61 -> 1.55 ms; the bare
+// copies of 52 MB each way in these chunks take 1.35 ms). 4 or 6 chunks: 1.59 / 1.57 ms; graded chunks
+// (small first and last): 1.66-1.71 ms.
 struct HostJob {
     int mode;
     double alpha, beta;

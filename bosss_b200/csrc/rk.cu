@@ -109,7 +109,8 @@ int bosss_b200_rk_steps_device(bosss_handle* h, int32_t stages, const double* a,
     cudaStream_t st = stream ? (cudaStream_t)stream : h->stream;
     // a graph costs its capture and instantiation (about 0.1 ms for four stages) once per call: it pays
     // from GRAPH_STEPS steps on; below, the launches of a step (about 3 us each) run ahead of their
-    // kernels just as well. GRAPHNOTE
+    // kernels just as well (3 RK4 steps, 17x12x9 cells, k = 2: 269 us with a graph, 259 us without, of
+    // them 258 us in kernels).
     constexpr int GRAPH_STEPS = 16;
     if (!use_graph || nsteps < GRAPH_STEPS) {
         for (int i = 0; i < nsteps; ++i) {

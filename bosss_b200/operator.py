@@ -467,6 +467,29 @@ class BlockMsrMatrix:
         return x, _report(r)
 
 
+def _address(a):
+    """Address of a tensor's or array's first element (an int: no ctypes object per argument)."""
+    return a.data_ptr() if hasattr(a, "data_ptr") else C.ptr(a)
+
+
+_raw_stream = None
+
+
+def _current_stream():
+    """Raw handle of the current torch stream (cudaStreamLegacy for torch's default stream). The
+    handle is looked up on every call, without the Stream object of ``current_stream()``, which
+    costs more than the launch it is for."""
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
+        get = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        if get is not None:
+            _raw_stream = lambda: get(torch.cuda.current_device())
+        else:
+            _raw_stream = lambda: torch.cuda.current_stream().cuda_stream
+    return _raw_stream() or C.CUDA_STREAM_LEGACY
+
+
 class Evaluator:
     """``IEvaluatorNonLin`` backed by one ``bosss_handle``."""
 
@@ -482,6 +505,7 @@ class Evaluator:
         C.check(C.lib().bosss_b200_create(ctypes.byref(self.desc), ctypes.byref(self.gdesc), ctypes.byref(opt),
                                           ctypes.byref(h)))
         self.handle = h
+        self._lib = C.lib()
         nd, nc, nq = ctypes.c_int64(), ctypes.c_int64(), ctypes.c_int32()
         C.check(C.lib().bosss_b200_get_sizes(h, ctypes.byref(nd), ctypes.byref(nc), ctypes.byref(nq)))
         self.n_domain, self.n_codomain, self.quad_nodes_1d = nd.value, nc.value, nq.value
@@ -518,9 +542,7 @@ class Evaluator:
     def _stream(self):
         """The current torch stream; torch's legacy default stream (handle 0) is passed as
         cudaStreamLegacy, since a NULL stream selects the handle's own stream."""
-        import torch
-        s = torch.cuda.current_stream().cuda_stream
-        return ctypes.c_void_p(s if s else C.CUDA_STREAM_LEGACY)
+        return _current_stream()
 
     def Evaluate(self, alpha, beta, output, U=None):
         """``output = beta*output + alpha*Op(U)``; ``U`` defaults to the bound domain
@@ -534,8 +556,10 @@ class Evaluator:
         if len(U) != self.n_domain or len(out) != self.n_codomain:
             raise C.BosssError(C.ERR_BAD_ARG, "wrong vector length")   # DifferentialOperator.cs:1590-1591
         if self._is_cuda(U):
-            C.check(C.lib().bosss_b200_evaluate_device(self.handle, alpha, beta, C.ptr(U), C.ptr(out),
-                                                       self.time, self._stream()))
+            rc = self._lib.bosss_b200_evaluate_device(self.handle, alpha, beta, _address(U), _address(out), self.time,
+                                                      _current_stream())
+            if rc:
+                C.check(rc)
         else:
             U = np.ascontiguousarray(U, dtype=np.float64)
             C.check(C.lib().bosss_b200_evaluate(self.handle, alpha, beta, C.ptr(U), C.ptr(out), self.time))
@@ -544,10 +568,13 @@ class Evaluator:
     def jvp(self, U, V, out=None):
         """J(U) V (directional derivative)."""
         if self._is_cuda(U):
-            import torch
-            out = torch.empty(self.n_codomain, dtype=torch.float64, device=U.device) if out is None else out
-            C.check(C.lib().bosss_b200_jvp_device(self.handle, C.ptr(U), C.ptr(V), C.ptr(out), self.time,
-                                                  self._stream()))
+            if out is None:
+                import torch
+                out = torch.empty(self.n_codomain, dtype=torch.float64, device=U.device)
+            rc = self._lib.bosss_b200_jvp_device(self.handle, _address(U), _address(V), _address(out), self.time,
+                                                 _current_stream())
+            if rc:
+                C.check(rc)
             return out
         U = np.ascontiguousarray(U, dtype=np.float64)
         V = np.ascontiguousarray(V, dtype=np.float64)
@@ -612,10 +639,13 @@ class Evaluator:
     def vjp(self, U, W, out=None):
         """J(U)^T W (adjoint product)."""
         if self._is_cuda(U):
-            import torch
-            out = torch.empty(self.n_domain, dtype=torch.float64, device=U.device) if out is None else out
-            C.check(C.lib().bosss_b200_vjp_device(self.handle, C.ptr(U), C.ptr(W), C.ptr(out), self.time,
-                                                  self._stream()))
+            if out is None:
+                import torch
+                out = torch.empty(self.n_domain, dtype=torch.float64, device=U.device)
+            rc = self._lib.bosss_b200_vjp_device(self.handle, _address(U), _address(W), _address(out), self.time,
+                                                 _current_stream())
+            if rc:
+                C.check(rc)
             return out
         U = np.ascontiguousarray(U, dtype=np.float64)
         W = np.ascontiguousarray(W, dtype=np.float64)

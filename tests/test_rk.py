@@ -171,3 +171,17 @@ def test_rk4_temporal_order_on_smooth_transport():
         assert 3.6 < rate < 4.4, (e1, e2, rate)
     finally:
         ev.Dispose()
+
+
+@pytest.mark.gpu
+def test_rk_captured_step_equals_plain_launches():
+    """Calls of 16 steps and more replay a captured step; the same bits as plain launches."""
+    import torch
+    pr = P.euler3d(n=4, k=1, seed=31)
+    with pr.evaluator() as ev:
+        Ug, Up = (torch.from_numpy(pr.U.copy()).cuda() for _ in range(2))
+        s = T.RungeKuttaScheme.RungeKutta1901()
+        T.RungeKutta(s, ev, None).PerformDevice(Ug, 1e-3, nsteps=17, use_graph=True)
+        T.RungeKutta(s, ev, None).PerformDevice(Up, 1e-3, nsteps=17, use_graph=False)
+        torch.cuda.synchronize()
+        assert torch.equal(Ug, Up)
