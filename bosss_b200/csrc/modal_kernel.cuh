@@ -45,6 +45,9 @@ struct ModalCfg {
     static constexpr int T = D == 2 ? 1 : (K == 4 ? 4 : K == 3 ? 2 : 1);
     static constexpr int MINB = D == 2 ? 4 : (K == 4 ? 1 : K == 3 ? 2 : K == 2 ? 4 : 8);
     static constexpr int NT = MODAL_CELLS * T;
+    // runs a warp copies at a time: few warps have several each (k = 2, 48^3: 29 -> 23 us), sixteen warps
+    // one or two (k = 4: four at a time 59 -> 71 us)
+    static constexpr int GRP = T == 1 ? 4 : T == 2 ? 2 : 1;
     // halo box of the largest tile: 4 x 4 x 8 cells in 3D, 8 x 16 in 2D, one zero slot, the results
     static constexpr int SLOTS = (D == 3 ? 6 * 6 * 10 : 10 * 18) + 1;
     // runs of cells to copy: per row of the tile its cells (with the halo cells that follow on), and
@@ -347,6 +350,7 @@ __device__ __forceinline__ void modal_tile(const EvalArgs& a, const Tables1D& T,
     constexpr int nw = NT >> 5;
     __shared__ ModalRun runs[C::RUNS];
     const int rA = e0 * e1, rB = 2 * e1, rC = (D == 3) ? 2 * e0 : 0, nrows = rA + rB + rC;
+    const int nlo = (o2 == 0 && per2) ? rA : 0, nhi = (o2 + e2 == n2 && per2) ? rA : 0;   // across the wrap
     for (int r = tid; r < nrows; r += NT) {
         int i0, i1;
         if (r < rA) {
@@ -370,26 +374,40 @@ __device__ __forceinline__ void modal_tile(const EvalArgs& a, const Tables1D& T,
             m1 = m1 < 0 ? m1 + n1 : m1 - n1;
         }
         const long long row = ((long long)m0 * n1 + m1) * n2;
-        ModalRun main{(row + o2) * NP, slot(i0, i1, 0), there ? e2 * NP : 0}, lo{0, 0, 0}, hi{0, 0, 0};
+        ModalRun main{(row + o2) * NP, slot(i0, i1, 0), there ? e2 * NP : 0};
         if (r < rA) {
             if (o2 > 0) {
                 main.src -= NP;
                 main.dst -= S;
                 main.n += NP;
-            } else if (per2) {
-                lo = ModalRun{(row + n2 - 1) * NP, slot(i0, i1, -1), NP};
+            } else if (nlo) {
+                runs[nrows + r] = ModalRun{(row + n2 - 1) * NP, slot(i0, i1, -1), NP};
             }
             if (o2 + e2 < n2) main.n += NP;
-            else if (per2) hi = ModalRun{row * NP, slot(i0, i1, e2), NP};
+            else if (nhi) runs[nrows + nlo + r] = ModalRun{row * NP, slot(i0, i1, e2), NP};
         }
-        runs[3 * r] = main;
-        runs[3 * r + 1] = lo;
-        runs[3 * r + 2] = hi;
+        runs[r] = main;
     }
     __syncthreads();
-    for (int r = warp; r < 3 * nrows; r += nw) {
-        const ModalRun q = runs[r];
-        for (int e = lane; e < q.n; e += 32) cp_async8(sm + q.dst + e + (S - NP) * (e / NP), in + q.src + e);
+    const int total = nrows + nlo + nhi;
+    for (int r = warp; r < total; r += C::GRP * nw) {   // several runs at a time: their addresses are independent
+        const double* src[C::GRP];
+        int dst[C::GRP], n[C::GRP], nmax = 0;
+#pragma unroll
+        for (int k = 0; k < C::GRP; ++k) {
+            const int rr = min(r + k * nw, total - 1);
+            const ModalRun q = runs[rr];
+            src[k] = in + q.src;
+            dst[k] = q.dst;
+            n[k] = r + k * nw < total ? q.n : 0;
+            nmax = max(nmax, n[k]);
+        }
+        for (int e = lane; e < nmax; e += 32) {
+            const int o = e + (S - NP) * (e / NP);
+#pragma unroll
+            for (int k = 0; k < C::GRP; ++k)
+                if (e < n[k]) cp_async8(sm + dst[k] + o, src[k] + e);
+        }
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
 
@@ -507,18 +525,29 @@ __device__ __forceinline__ void modal_tile(const EvalArgs& a, const Tables1D& T,
         }
     }
     // ---- results stored in runs of cells
-    for (int r = warp; r < e0 * e1; r += nw) {
-        const int i0 = r / e1, i1 = r - i0 * e1;
-        const long long row = ((long long)(o0 + i0) * n1 + (o1 + i1)) * n2 + o2;
-        const double* src = res + ((i0 * b1 + i1) * b2) * S;
-        double* dst = out + row * NP;
-        const bool whole = row >= a.cbeg && row + e2 <= a.cend;
+    for (int r = warp; r < rA; r += C::GRP * nw) {
+        const double* src[C::GRP];
+        double* dst[C::GRP];
+        long long first[C::GRP];
+#pragma unroll
+        for (int k = 0; k < C::GRP; ++k) {
+            const int rr = min(r + k * nw, rA - 1);
+            const ModalRun q = runs[rr];
+            const long long at = q.src + (o2 > 0 ? NP : 0);   // the row's own cells
+            const int i0 = rr / e1, i1 = rr - i0 * e1;
+            src[k] = res + ((i0 * b1 + i1) * b2) * S;
+            dst[k] = out + at;
+            first[k] = at / NP;
+        }
         for (int e = lane; e < e2 * NP; e += 32) {
-            const int c = e / NP;
-            if (!whole && (row + c < a.cbeg || row + c >= a.cend)) continue;
-            const double v = src[e + c * (S - NP)];
-            if (MODE == MODE_RES) dst[e] = (beta == 0.0) ? alpha * v : beta * dst[e] + alpha * v;
-            else dst[e] = v;
+            const int c = e / NP, o = e + c * (S - NP);
+#pragma unroll
+            for (int k = 0; k < C::GRP; ++k) {
+                if (r + k * nw >= rA || first[k] + c < a.cbeg || first[k] + c >= a.cend) continue;
+                const double v = src[k][o];
+                if (MODE == MODE_RES) dst[k][e] = (beta == 0.0) ? alpha * v : beta * dst[k][e] + alpha * v;
+                else dst[k][e] = v;
+            }
         }
     }
 }
