@@ -482,11 +482,28 @@ struct bosss_pmg {
         for (void* p : owned) cudaFree(p);
         if (stream) cudaStreamDestroy(stream);
     }
-    double* alloc(size_t n) {
+    // all arrays come from one reserved block: some 25 allocations per setup took longer than its kernels
+    double* block = nullptr;
+    size_t left = 0;
+    static size_t padded(size_t n) { return (std::max<size_t>(n, 1) + 31) / 32 * 32; }
+    bool reserve(size_t n) {
         void* p = nullptr;
-        if (cudaMalloc(&p, sizeof(double) * std::max<size_t>(n, 1)) != cudaSuccess) return nullptr;
+        if (cudaMalloc(&p, sizeof(double) * n) != cudaSuccess) return false;
         owned.push_back(p);
-        return (double*)p;
+        block = (double*)p;
+        left = n;
+        return true;
+    }
+    double* alloc(size_t n) {
+        n = padded(n);
+        if (n > left) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        double* p = block;
+        block += n;
+        left -= n;
+        return p;
     }
 
     // the structured part of the cycle from level l: input H[l].b, output in H[l].x
@@ -570,6 +587,42 @@ int pmg_create(const bosss_handle* h, const bosss_bsr* A, bosss_pmg** out) {
     cudaError_t e = cudaStreamCreateWithFlags(&M->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return cuda_bail(e, "stream");
     cudaStream_t s = M->stream;
+    // the structured levels' geometry, then one block for every array
+    {
+        bosss_pmg::HLevel L;
+        for (int d = 0; d < 3; ++d) {
+            L.g.n[d] = d < g.D ? g.n[d] : 1;
+            L.g.per[d] = d < g.D ? g.periodic[d] : 0;
+            L.g.stride[d] = d < g.D ? (int)g.stride[d] : 1;
+        }
+        L.g.N = g.J;
+        M->H.push_back(L);
+    }
+    while (true) {
+        const SGeom& f = M->H.back().g;
+        if (f.N <= COARSE_MAX || (f.n[0] == 1 && f.n[1] == 1 && f.n[2] == 1)) break;
+        bosss_pmg::HLevel C;
+        for (int d = 0; d < 3; ++d) {
+            C.g.n[d] = (f.n[d] + 1) / 2;
+            C.g.per[d] = f.per[d];
+        }
+        C.g.stride[2] = 1;
+        C.g.stride[1] = C.g.n[2];
+        C.g.stride[0] = C.g.n[1] * C.g.n[2];
+        C.g.N = (long long)C.g.n[0] * C.g.n[1] * C.g.n[2];
+        M->H.push_back(C);
+    }
+    {
+        auto pad = [](size_t n) { return bosss_pmg::padded(n); };
+        size_t total = pad((size_t)g.J + 1) + pad(((size_t)A->nnzb + 1) / 2) + 2 * pad((size_t)g.J * m0) + pad(1);
+        for (int k = h->K; k >= 1; --k) {
+            const size_t m = np_of(h->D, k), nx = (size_t)g.J * m;
+            total += pad((size_t)A->nnzb * m * m) + pad(nx * m) + pad(nx) * (k == h->K ? 1 : 3);
+        }
+        for (const auto& L : M->H) total += pad((size_t)NS * L.g.N) + 3 * pad((size_t)L.g.N);
+        if (M->H.back().g.N <= COARSE_MAX) total += 2 * pad((size_t)(M->H.back().g.N * M->H.back().g.N));
+        if (!M->reserve(total)) return cuda_bail(cudaErrorMemoryAllocation, "alloc");
+    }
     // the pattern (self first, then face neighbours) is shared by every p-level
     M->rowptr = (long long*)M->alloc((size_t)g.J + 1);
     M->colidx = (int*)M->alloc(((size_t)A->nnzb + 1) / 2);
@@ -605,30 +658,6 @@ int pmg_create(const bosss_handle* h, const bosss_bsr* A, bosss_pmg** out) {
         M->P.push_back(L);
     }
     // structured levels: the piecewise-constant level of the grid, then aggregates
-    {
-        bosss_pmg::HLevel L;
-        for (int d = 0; d < 3; ++d) {
-            L.g.n[d] = d < g.D ? g.n[d] : 1;
-            L.g.per[d] = d < g.D ? g.periodic[d] : 0;
-            L.g.stride[d] = d < g.D ? (int)g.stride[d] : 1;
-        }
-        L.g.N = g.J;
-        M->H.push_back(L);
-    }
-    while (true) {
-        const SGeom& f = M->H.back().g;
-        if (f.N <= COARSE_MAX || (f.n[0] == 1 && f.n[1] == 1 && f.n[2] == 1)) break;
-        bosss_pmg::HLevel C;
-        for (int d = 0; d < 3; ++d) {
-            C.g.n[d] = (f.n[d] + 1) / 2;
-            C.g.per[d] = f.per[d];
-        }
-        C.g.stride[2] = 1;
-        C.g.stride[1] = C.g.n[2];
-        C.g.stride[0] = C.g.n[1] * C.g.n[2];
-        C.g.N = (long long)C.g.n[0] * C.g.n[1] * C.g.n[2];
-        M->H.push_back(C);
-    }
     for (auto& L : M->H) {
         L.st = M->alloc((size_t)NS * L.g.N);
         L.b = M->alloc((size_t)L.g.N);

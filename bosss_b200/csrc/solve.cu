@@ -211,13 +211,14 @@ static int assemble(bosss_handle* h, const double* U_dev, double time, bosss_bsr
     if (e == cudaSuccess) e = cudaMemsetAsync(A->d_vals, 0, sizeof(double) * bs * ci.size(), s);
     double *V = nullptr, *JV = nullptr;
     int* colour = nullptr;   // of every cell: found once, read by all probes and scatters
-    if (e == cudaSuccess) e = cudaMalloc(&V, sizeof(double) * h->ndom);
-    if (e == cudaSuccess) e = cudaMalloc(&JV, sizeof(double) * h->ncod);
-    if (e == cudaSuccess) e = cudaMalloc(&colour, sizeof(int) * std::max<int64_t>(g.J, 1));
+    const size_t nV = ((size_t)h->ndom + 31) / 32 * 32, nJV = ((size_t)h->ncod + 31) / 32 * 32;
+    if (e == cudaSuccess) e = cudaMalloc(&V, sizeof(double) * (nV + nJV) + sizeof(int) * (size_t)g.J);   // all three
+    if (e == cudaSuccess) {
+        JV = V + nV;
+        colour = (int*)(JV + nJV);
+    }
     if (e != cudaSuccess) {
         cudaFree(V);
-        cudaFree(JV);
-        cudaFree(colour);
         return bail(e);
     }
     const Colouring c = make_colouring(g);
@@ -228,8 +229,6 @@ static int assemble(bosss_handle* h, const double* U_dev, double time, bosss_bsr
             int rc = run_mode(h, MODE_JVP, 1.0, 0.0, U_dev, V, JV, time, s);
             if (rc) {
                 cudaFree(V);
-                cudaFree(JV);
-                cudaFree(colour);
                 bosss_b200_bsr_destroy(A);
                 return rc;
             }
@@ -239,8 +238,6 @@ static int assemble(bosss_handle* h, const double* U_dev, double time, bosss_bsr
         }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     cudaFree(V);
-    cudaFree(JV);
-    cudaFree(colour);
     if (e != cudaSuccess) return bail(e);
     *out = A;
     return BOSSS_OK;
@@ -330,22 +327,24 @@ struct KrylovWork {
     double* partials = nullptr;
     double* hbuf = nullptr;
     double* pinned = nullptr;   // host slots of the lagged residual checks
+    void* block = nullptr;      // one allocation for all device arrays (cudaMalloc and cudaFree synchronise)
     ~KrylovWork() {
-        cudaFree(V);
-        cudaFree(w);
-        cudaFree(z);
-        cudaFree(partials);
-        cudaFree(hbuf);
+        cudaFree(block);
         if (pinned) cudaFreeHost(pinned);
     }
     cudaError_t alloc(long long n, int m) {
-        cudaError_t e = cudaMalloc(&V, sizeof(T) * (size_t)(m + 1) * n);
-        if (e == cudaSuccess) e = cudaMalloc(&w, sizeof(T) * n);
-        if (e == cudaSuccess) e = cudaMalloc(&z, sizeof(T) * n);
-        if (e == cudaSuccess) e = cudaMalloc(&partials, sizeof(double) * RED_BLOCKS * (m + 1));
-        if (e == cudaSuccess) e = cudaMalloc(&hbuf, sizeof(double) * gmres_dev_doubles(m));
-        if (e == cudaSuccess) e = cudaMallocHost(&pinned, sizeof(double) * 8);
-        return e;
+        auto up = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
+        const size_t bV = up(sizeof(T) * (size_t)(m + 1) * n), bn = up(sizeof(T) * n);
+        const size_t bp = up(sizeof(double) * RED_BLOCKS * (m + 1)), bh = up(sizeof(double) * gmres_dev_doubles(m));
+        cudaError_t e = cudaMalloc(&block, bV + 2 * bn + bp + bh);
+        if (e != cudaSuccess) return e;
+        char* q = (char*)block;
+        V = (T*)q;
+        w = (T*)(q + bV);
+        z = (T*)(q + bV + bn);
+        partials = (double*)(q + bV + 2 * bn);
+        hbuf = (double*)(q + bV + 2 * bn + bp);
+        return cudaMallocHost(&pinned, sizeof(double) * 8);
     }
 };
 
@@ -449,18 +448,18 @@ int bosss_b200_newton_solve(bosss_handle* h, double* U, double time, const bosss
     KrylovWork<double> kw;
     auto cleanup = [&]() {
         pmg_destroy(mg);
-        cudaFree(dU);
-        cudaFree(dR);
-        cudaFree(dX);
-        cudaFree(dT);
-        cudaFree(dW);
+        cudaFree(dU);   // start of the block
         cudaFree(dinv);
     };
-    cudaError_t e = cudaMalloc(&dU, sizeof(double) * n);
-    if (e == cudaSuccess) e = cudaMalloc(&dR, sizeof(double) * n);
-    if (e == cudaSuccess) e = cudaMalloc(&dX, sizeof(double) * n);
-    if (e == cudaSuccess) e = cudaMalloc(&dT, sizeof(double) * n);
-    if (e == cudaSuccess) e = cudaMalloc(&dW, sizeof(double) * n);
+    // one allocation for the five vectors
+    const long long nv = (n + 31) / 32 * 32;
+    cudaError_t e = cudaMalloc(&dU, sizeof(double) * 5 * nv);
+    if (e == cudaSuccess) {
+        dR = dU + nv;
+        dX = dR + nv;
+        dT = dX + nv;
+        dW = dT + nv;
+    }
     if (e == cudaSuccess) e = kw.alloc(n, o.restart);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dU, U, sizeof(double) * n, cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) {

@@ -145,11 +145,12 @@ constexpr int RED_BLOCKS = 296;   // 2 x 148 SMs
 constexpr int RED_THREADS = 512;
 constexpr int MDOT_CH = 8;        // vectors per pass of the multi-dot
 
-// <V_k, w> for k in [k0, min(k0 + MDOT_CH, m)), w read once per pass: one FP64 partial per
+// <V_k, w> for k in [k0, min(k0 + MDOT_CH, m)), k0 = MDOT_CH * blockIdx.y, w read once per pass: one FP64 partial per
 // (k, block) in partials[k * RED_BLOCKS + block]
 template <class T>
-__global__ void __launch_bounds__(RED_THREADS) k_mdot(long long n, int k0, int m, const T* __restrict__ V, long long ldv,
+__global__ void __launch_bounds__(RED_THREADS) k_mdot(long long n, int m, const T* __restrict__ V, long long ldv,
                                                      const T* __restrict__ w, double* __restrict__ partials) {
+    const int k0 = MDOT_CH * blockIdx.y;
     double acc[MDOT_CH];
 #pragma unroll
     for (int c = 0; c < MDOT_CH; ++c) acc[c] = 0.0;
@@ -286,13 +287,12 @@ GmresResult gmres(long long n, const std::function<cudaError_t(const T*, T*)>& a
     GmresDev dv(work, m);
     // sum_k (k < cnt) <V_k, vec> -> out[k] on the device
     auto mdot = [&](int cnt, const T* vec, double* out) {
-        for (int k0 = 0; k0 < cnt; k0 += MDOT_CH)
-            k_mdot<T><<<RED_BLOCKS, RED_THREADS, 0, s>>>(n, k0, cnt, V, n, vec, partials);
+        k_mdot<T><<<dim3(RED_BLOCKS, (cnt + MDOT_CH - 1) / MDOT_CH), RED_THREADS, 0, s>>>(n, cnt, V, n, vec, partials);
         k_finish_partials<<<cnt, 256, 0, s>>>(partials, out);
         chk(cudaGetLastError());
     };
     auto norm2_dev = [&](const T* a) {   // ||a||^2 -> sc[0]
-        k_mdot<T><<<RED_BLOCKS, RED_THREADS, 0, s>>>(n, 0, 1, a, n, a, partials);
+        k_mdot<T><<<RED_BLOCKS, RED_THREADS, 0, s>>>(n, 1, a, n, a, partials);
         k_finish_partials<<<1, 256, 0, s>>>(partials, dv.sc);
         chk(cudaGetLastError());
     };
