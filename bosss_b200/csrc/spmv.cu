@@ -54,11 +54,47 @@ __global__ void k_to_ell(long long nbr, int br, int bc, int w, const long long* 
     }
 }
 
-template <int BC>
-__global__ void __launch_bounds__(256) k_ell_spmv(long long nbr, int br, int bc_rt, int w, const int* __restrict__ ell_col,
+// G block slots are in flight at a time: a row's loads then take two or three memory latencies
+// instead of one or two per slot, which is what the last wave of warps waits for (values alone at
+// full occupancy would keep the memory busy either way)
+template <int BC, int G>
+__global__ void __launch_bounds__(256) k_ell_spmv(long long nbr, int br, int w, const int* __restrict__ ell_col,
                                                   const double* __restrict__ ell_vals, const double* __restrict__ x,
                                                   double alpha, double beta, double* __restrict__ y) {
-    const int bc = BC > 0 ? BC : bc_rt;
+    const long long nrows = nbr * br;
+    for (long long row = blockIdx.x * (long long)blockDim.x + threadIdx.x; row < nrows;
+         row += (long long)gridDim.x * blockDim.x) {
+        const long long i = row / br;
+        const double* v = ell_vals + (row / SLICE) * w * BC * SLICE + (row % SLICE);
+        double acc = 0.0;
+        for (int s = 0; s < w; s += G) {
+            double a[G][BC];
+            long long col[G];
+#pragma unroll
+            for (int k = 0; k < G; ++k)
+                if (s + k < w) col[k] = ell_col[(long long)(s + k) * nbr + i];
+#pragma unroll
+            for (int k = 0; k < G; ++k)
+                if (s + k < w) {
+#pragma unroll
+                    for (int c = 0; c < BC; ++c) a[k][c] = __ldcs(v + ((s + k) * BC + c) * SLICE);
+                }
+#pragma unroll
+            for (int k = 0; k < G; ++k)
+                if (s + k < w) {
+                    const double* xb = x + col[k] * BC;
+#pragma unroll
+                    for (int c = 0; c < BC; ++c) acc += a[k][c] * __ldg(xb + c);
+                }
+        }
+        y[row] = (beta == 0.0) ? alpha * acc : beta * y[row] + alpha * acc;
+    }
+}
+
+// any block width
+__global__ void __launch_bounds__(256) k_ell_spmv_any(long long nbr, int br, int bc, int w, const int* __restrict__ ell_col,
+                                                      const double* __restrict__ ell_vals, const double* __restrict__ x,
+                                                      double alpha, double beta, double* __restrict__ y) {
     const long long nrows = nbr * br;
     for (long long row = blockIdx.x * (long long)blockDim.x + threadIdx.x; row < nrows;
          row += (long long)gridDim.x * blockDim.x) {
@@ -68,12 +104,7 @@ __global__ void __launch_bounds__(256) k_ell_spmv(long long nbr, int br, int bc_
         for (int s = 0; s < w; ++s) {
             const double* xb = x + (long long)ell_col[(long long)s * nbr + i] * bc;
             const double* vs = v + (long long)s * bc * SLICE;
-            if (BC > 0) {
-#pragma unroll
-                for (int c = 0; c < BC; ++c) acc += __ldcs(vs + c * SLICE) * __ldg(xb + c);
-            } else {
-                for (int c = 0; c < bc; ++c) acc += __ldcs(vs + c * SLICE) * __ldg(xb + c);
-            }
+            for (int c = 0; c < bc; ++c) acc += __ldcs(vs + c * SLICE) * __ldg(xb + c);
         }
         y[row] = (beta == 0.0) ? alpha * acc : beta * y[row] + alpha * acc;
     }
@@ -143,12 +174,26 @@ int bsr_spmv(bosss_bsr* A, double alpha, const double* x, double beta, double* y
     if (rc) return rc;
     const int grid = grid_for(nrows);
     if (A->ell_w > 0) {
+        // slots in flight per row (hex patterns, B200, L2 flushed): two at most sizes (10 x 10 blocks, 48^3 cells
+        // 109.5 -> 104.4 us, 34^3 51.2 -> 43.0; 20 x 20, 26^3 79.9 -> 68.4; 35 x 35, 20^3: one 97.3, two 135.2).
+        // Below 512 rows per SM nothing but the chain of loads counts: more (10 x 10, 12^3 22.5 -> 10.3 us
+        // with four, 13.3 with two; 35 x 35, 8^3 47.1 -> 22.5 with two)
+        const bool few = nrows < 148LL * 512;
         switch (A->bc) {
-            case 4: k_ell_spmv<4><<<grid, 256, 0, s>>>(A->nbr, A->br, A->bc, A->ell_w, A->d_ell_col, A->d_ell_vals, x, alpha, beta, y); break;
-            case 10: k_ell_spmv<10><<<grid, 256, 0, s>>>(A->nbr, A->br, A->bc, A->ell_w, A->d_ell_col, A->d_ell_vals, x, alpha, beta, y); break;
-            case 20: k_ell_spmv<20><<<grid, 256, 0, s>>>(A->nbr, A->br, A->bc, A->ell_w, A->d_ell_col, A->d_ell_vals, x, alpha, beta, y); break;
-            case 35: k_ell_spmv<35><<<grid, 256, 0, s>>>(A->nbr, A->br, A->bc, A->ell_w, A->d_ell_col, A->d_ell_vals, x, alpha, beta, y); break;
-            default: k_ell_spmv<0><<<grid, 256, 0, s>>>(A->nbr, A->br, A->bc, A->ell_w, A->d_ell_col, A->d_ell_vals, x, alpha, beta, y); break;
+#define BOSSS_SPMV(BC, G) \
+    case BC: k_ell_spmv<BC, G><<<grid, 256, 0, s>>>(A->nbr, A->br, A->ell_w, A->d_ell_col, A->d_ell_vals, x, alpha, beta, y); break;
+            BOSSS_SPMV(4, 2)
+            case 10:
+                if (few) k_ell_spmv<10, 4><<<grid, 256, 0, s>>>(A->nbr, A->br, A->ell_w, A->d_ell_col, A->d_ell_vals, x, alpha, beta, y);
+                else k_ell_spmv<10, 2><<<grid, 256, 0, s>>>(A->nbr, A->br, A->ell_w, A->d_ell_col, A->d_ell_vals, x, alpha, beta, y);
+                break;
+            BOSSS_SPMV(20, 2)
+            case 35:
+                if (few) k_ell_spmv<35, 2><<<grid, 256, 0, s>>>(A->nbr, A->br, A->ell_w, A->d_ell_col, A->d_ell_vals, x, alpha, beta, y);
+                else k_ell_spmv<35, 1><<<grid, 256, 0, s>>>(A->nbr, A->br, A->ell_w, A->d_ell_col, A->d_ell_vals, x, alpha, beta, y);
+                break;
+#undef BOSSS_SPMV
+            default: k_ell_spmv_any<<<grid, 256, 0, s>>>(A->nbr, A->br, A->bc, A->ell_w, A->d_ell_col, A->d_ell_vals, x, alpha, beta, y);
         }
     } else {
         k_bsr_spmv<<<grid, 256, 0, s>>>(A->nbr, A->br, A->bc, (const long long*)A->d_rowptr, A->d_colidx, A->d_vals,
