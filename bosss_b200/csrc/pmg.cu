@@ -308,13 +308,39 @@ __global__ void k_resid(unsigned n, int mr, int mo, const long long* __restrict_
         const unsigned j = t / mo, r = t - j * mo;
         double acc = b[(long long)j * m + r];
         const long long b0 = rowptr[j], b1 = rowptr[j + 1];
-        for (long long bb = b0; bb < b1; ++bb) {
-            const double* blk = vals + bb * (long long)m * m + r;
-            const double* xb = x + (long long)colidx[bb] * m;
-            double s = 0.0;
+        if constexpr (M == 0) {
+            for (long long bb = b0; bb < b1; ++bb) {
+                const double* blk = vals + bb * (long long)m * m + r;
+                const double* xb = x + (long long)colidx[bb] * m;
+                double s = 0.0;
+                for (int c = 0; c < m; ++c) s += blk[(long long)c * m] * xb[c];
+                acc -= s;
+            }
+        } else {
+            constexpr int G = M <= 6 ? 4 : M <= 10 ? 2 : 1;   // blocks of the row in flight
+            for (long long bb = b0; bb < b1; bb += G) {
+                double a[G][M];
+                long long col[G];
 #pragma unroll
-            for (int c = 0; c < m; ++c) s += blk[(long long)c * m] * xb[c];
-            acc -= s;
+                for (int k = 0; k < G; ++k)
+                    if (bb + k < b1) col[k] = colidx[bb + k];
+#pragma unroll
+                for (int k = 0; k < G; ++k)
+                    if (bb + k < b1) {
+                        const double* blk = vals + (bb + k) * M * M + r;
+#pragma unroll
+                        for (int c = 0; c < M; ++c) a[k][c] = blk[c * M];
+                    }
+#pragma unroll
+                for (int k = 0; k < G; ++k)
+                    if (bb + k < b1) {
+                        const double* xb = x + col[k] * M;
+                        double s = 0.0;
+#pragma unroll
+                        for (int c = 0; c < M; ++c) s += a[k][c] * xb[c];
+                        acc -= s;
+                    }
+            }
         }
         out[t] = acc;
     }

@@ -19,6 +19,17 @@ ModalTile sip_tiling(const EvalArgs& a) {
     const long long plane = (long long)n1 * n2;
     const int s0 = (int)(a.cbeg / plane), s1 = (int)std::min<long long>(n0, (a.cend + plane - 1) / plane);
     const int m0 = std::max(1, s1 - s0);
+    // the extents depend on the sizes alone: the last ones found on this thread are kept
+    struct Memo {
+        int m0 = 0, n1 = 0, n2 = 0;
+        ModalTile t{};
+    };
+    static thread_local Memo memo;
+    if (memo.m0 == m0 && memo.n1 == n1 && memo.n2 == n2) {
+        ModalTile t = memo.t;
+        t.s0 = s0;
+        return t;
+    }
     ModalTile best{};
     double bc = 1e300;
     const int ext[] = {1, 2, 3, 4, 5, 6, 8};
@@ -45,8 +56,12 @@ ModalTile sip_tiling(const EvalArgs& a) {
                     best.t[2] = (int)t2;
                 }
             }
-    best.s0 = s0;
     best.ncell = best.b[0] * best.b[1] * best.b[2];
+    memo.m0 = m0;
+    memo.n1 = n1;
+    memo.n2 = n2;
+    memo.t = best;
+    best.s0 = s0;
     return best;
 }
 

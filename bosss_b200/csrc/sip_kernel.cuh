@@ -30,11 +30,13 @@ struct SipCfg {
     static constexpr int QV = Q < 2 * K ? Q : 2 * K;
     static constexpr int NG = MODE == MODE_RES ? 1 : 2;
     static constexpr int S = NP | 1;
-    static constexpr int NT = 256;
-    // largest block, its halo box and its faces per direction
-    static constexpr int CELLS = K == 1 ? 128 : K == 2 ? 64 : K == 3 ? 48 : 32;
-    static constexpr int SLOTS = K == 1 ? 360 : K == 2 ? 216 : K == 3 ? 180 : 144;
-    static constexpr int FACES = K == 1 ? 160 : K == 2 ? 80 : K == 3 ? 64 : 48;
+    // threads, largest block, its halo box and its faces per direction (swept on B200; k = 4 residual at
+    // 18^3: two CTAs of 192 threads with 16 cells 82 us, one of 256 with 32 cells 92 us)
+    static constexpr bool R4 = K == 4 && MODE == MODE_RES;
+    static constexpr int NT = R4 ? 192 : 256;
+    static constexpr int CELLS = K == 1 ? 128 : K == 2 ? 64 : K == 3 ? 48 : R4 ? 16 : 32;
+    static constexpr int SLOTS = K == 1 ? 360 : K == 2 ? 216 : K == 3 ? 180 : R4 ? 96 : 144;
+    static constexpr int FACES = K == 1 ? 160 : K == 2 ? 80 : K == 3 ? 64 : R4 ? 24 : 48;
     static constexpr int FST = FACES | 1, CST = CELLS | 1;
     static constexpr int NA = MODE == MODE_VJP ? 4 : 3;      // face results: g, G_A, G_B / g_A, G_A, g_B, G_B
     static constexpr int TR = 4 * NG * NPAIR;                // traces of a face
@@ -45,9 +47,6 @@ struct SipCfg {
     static constexpr size_t SMEM = sizeof(double) * (O_WORK + WORK);
     static constexpr int MINB = SMEM <= 112 * 1024 ? 2 : 1;
 };
-
-__device__ constexpr double kSipE[5] = {0.70710678118654752440, 1.22474487139158904910, 1.58113883008418966600,
-                                        1.87082869338697069279, 2.12132034355964257320};
 
 template <int DIR>
 __device__ __forceinline__ constexpr int sip_mode(int m, int p, int r) {
@@ -97,23 +96,21 @@ __device__ __forceinline__ void sip_rows(const double* c, const double* Ay, cons
 }
 
 template <int K, int Q, int MODE, int DIR>
-__device__ __forceinline__ void sip_traces(const EvalArgs& a, const TileGeom& G, const double* coef, double* tr, int fd0,
-                                           int fd1, int fd2) {
+__device__ __forceinline__ void sip_traces(const EvalArgs& a, const TileGeom& G, const double* coef, double* tr, int fd1,
+                                           int fd2, int nf, int t) {
     using C = SipCfg<K, Q, MODE>;
-    const int nf = fd0 * fd1 * fd2, md = G.mem(DIR);
+    const int md = G.mem(DIR);
     const double sc = a.g.scaling, scn = a.g.scaling * a.g.twoh[DIR];
-    for (int t = threadIdx.x; t < 2 * C::NG * nf; t += C::NT) {
+    {
         const int gs = t / nf, f = t - gs * nf;          // gs = group * 2 + side
         const int side = gs & 1, grp = gs >> 1;
         const int f2 = f % fd2, fq = f / fd2, f1 = fq % fd1, f0 = fq / fd1;
-        int i[3] = {f0, f1, f2};
         const int at = (md == 0 ? f0 : md == 1 ? f1 : f2) - 1 + side;   // tile coordinate of the cell
         const int gi = (md == 0 ? G.o[0] : md == 1 ? G.o[1] : G.o[2]) + at;
         const int nn = md == 0 ? G.n[0] : md == 1 ? G.n[1] : G.n[2];
         const int pp = md == 0 ? G.per[0] : md == 1 ? G.per[1] : G.per[2];
         const bool there = (gi >= 0 && gi < nn) || pp;
         const int sl = md == 0 ? G.slot(at, f1, f2) : md == 1 ? G.slot(f0, at, f2) : G.slot(f0, f1, at);
-        (void)i;
         const double* c = coef + (size_t)grp * C::SLOTS * C::S + sl * C::S;
         double* o = tr + (size_t)gs * 2 * C::NPAIR * C::FST + f;
         int pr = 0;
@@ -126,7 +123,7 @@ __device__ __forceinline__ void sip_traces(const EvalArgs& a, const TileGeom& G,
 #pragma unroll
                     for (int m = 0; m <= K - p - r; ++m) {
                         const double v = c[sip_mode<DIR>(m, p, r)];
-                        const double E = kSipE[m], F = kSipE[m] * (0.5 * m * (m + 1));
+                        const double E = a.tab.e[1][m], F = a.tab.de[1][m];   // L_m(1), L_m'(1)
                         if (m & 1) {
                             vo += v * E;
                             dq += v * F;
@@ -336,45 +333,45 @@ __device__ __forceinline__ void sip_face_rows(const EvalArgs& a, const TileGeom&
     }
 }
 
-// (cell, pencil) threads: rows of the cell's two faces contracted over the second direction and
-// multiplied with the traces of the test functions
+// one (cell, pencil): rows of the cell's two faces contracted over the second direction and multiplied
+// with the traces of the test functions. The pencil is a constant of the branch (the same for a warp
+// where the cell count is a multiple of 32)
 template <int K, int Q, int MODE, int DIR>
 __device__ __forceinline__ void sip_face_add(const EvalArgs& a, const TileGeom& G, const double* rows, double* R, int ncell,
-                                             int b1, int b2, int fd1, int fd2) {
+                                             int b1, int b2, int fd1, int fd2, int t) {
     using C = SipCfg<K, Q, MODE>;
     const Tables1D& T = a.tab;
     const int md = G.mem(DIR);
     const int fs = md == 0 ? fd1 * fd2 : md == 1 ? fd2 : 1;   // face stride along DIR
-    for (int t = threadIdx.x; t < C::NPAIR * ncell; t += C::NT) {
-        const int pr = t / ncell, c = t - pr * ncell;
-        const int l2 = c % b2, lq = c / b2, l1 = lq % b1, l0 = lq / b1;
-        if (l0 >= G.e[0] || l1 >= G.e[1] || l2 >= G.e[2]) continue;
-        const int fl = (l0 * fd1 + l1) * fd2 + l2, fu = fl + fs;
-        int p = 0, r = pr;   // pair (p, r): r runs fastest, K + 1 - p entries per p
-        while (r > K - p) {
-            r -= K + 1 - p;
-            ++p;
-        }
-        constexpr int iB = MODE == MODE_VJP ? 2 : 0, iGB = MODE == MODE_VJP ? 3 : 2;
-        double gu = 0.0, Gu = 0.0, gl = 0.0, Gl = 0.0;
+    const int pr = t / ncell, c = t - pr * ncell;
+    const int l2 = c % b2, lq = c / b2, l1 = lq % b1, l0 = lq / b1;
+    if (l0 >= G.e[0] || l1 >= G.e[1] || l2 >= G.e[2]) return;
+    const int fl = (l0 * fd1 + l1) * fd2 + l2, fu = fl + fs;
+    constexpr int iB = MODE == MODE_VJP ? 2 : 0, iGB = MODE == MODE_VJP ? 3 : 2;
+    int i = 0;
 #pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            const double A = T.A[q][r];
-            gu += rows[((0 * (K + 1) + p) * Q + q) * C::FST + fu] * A;
-            Gu += rows[((1 * (K + 1) + p) * Q + q) * C::FST + fu] * A;
-            gl += rows[((iB * (K + 1) + p) * Q + q) * C::FST + fl] * A;
-            Gl += rows[((iGB * (K + 1) + p) * Q + q) * C::FST + fl] * A;
-        }
-        if (MODE != MODE_VJP) gl = -gl;
-        const double gs = gu + gl, gd = gu - gl, Gs = Gu + Gl, Gd = Gu - Gl;
+    for (int p = 0; p <= K; ++p)
 #pragma unroll
-        for (int m = 0; m <= K; ++m)
-            if (m <= K - p - r) {
-                const int n = sip_mode<DIR>(m, p, r);
-                const double E = kSipE[m], F = kSipE[m] * (0.5 * m * (m + 1));
-                R[n * C::CST + c] += ((m & 1) ? gd : gs) * E + ((m & 1) ? Gs : Gd) * F;
+        for (int r = 0; r <= K - p; ++r, ++i) {
+            if (pr != i) continue;
+            double gu = 0.0, Gu = 0.0, gl = 0.0, Gl = 0.0;
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                gu += rows[((0 * (K + 1) + p) * Q + q) * C::FST + fu] * T.A[q][r];
+                Gu += rows[((1 * (K + 1) + p) * Q + q) * C::FST + fu] * T.A[q][r];
+                gl += rows[((iB * (K + 1) + p) * Q + q) * C::FST + fl] * T.A[q][r];
+                Gl += rows[((iGB * (K + 1) + p) * Q + q) * C::FST + fl] * T.A[q][r];
             }
-    }
+            if (MODE != MODE_VJP) gl = -gl;
+            const double gs = gu + gl, gd = gu - gl, Gs = Gu + Gl, Gd = Gu - Gl;
+#pragma unroll
+            for (int m = 0; m <= K - p - r; ++m) {
+                const int n = sip_mode<DIR>(m, p, r);
+                double v = ((m & 1) ? gd : gs) * T.e[1][m];
+                if (m > 0) v += ((m & 1) ? Gs : Gd) * T.de[1][m];
+                R[n * C::CST + c] += v;
+            }
+        }
 }
 
 template <int K, int Q, int MODE>
@@ -535,17 +532,31 @@ k_sip(const __grid_constant__ EvalArgs a, const __grid_constant__ Tables1D V, co
     };
     auto direction = [&](auto dirc) {
         constexpr int DIR = decltype(dirc)::value;
-        int f0, f1, f2;
+        int f0, f1, f2, p0 = 0, p1 = 0, p2 = 0;
         dims(DIR, f0, f1, f2);
-        sip_traces<K, Q, MODE, DIR>(a, G, coef, tr, f0, f1, f2);
+        if constexpr (DIR > 0) dims(DIR - 1, p0, p1, p2);
+        // this direction's traces, and the previous direction's faces into the cells
+        const int nf = f0 * f1 * f2, ntr = 2 * C::NG * nf, nadd = DIR > 0 ? C::NPAIR * ncell : 0;
+        for (int t = threadIdx.x; t < ntr + nadd; t += C::NT) {
+            if (t < nadd) {
+                if constexpr (DIR > 0) sip_face_add<K, Q, MODE, DIR - 1>(a, G, rows, R, ncell, b1, b2, p1, p2, t);
+            } else {
+                sip_traces<K, Q, MODE, DIR>(a, G, coef, tr, f1, f2, nf, t - nadd);
+            }
+        }
         __syncthreads();
         sip_face_rows<K, Q, MODE, DIR>(a, G, tr, rows, f0, f1, f2);
         __syncthreads();
-        sip_face_add<K, Q, MODE, DIR>(a, G, rows, R, ncell, b1, b2, f1, f2);   // overlaps the next traces
     };
     direction(std::integral_constant<int, 0>{});
     direction(std::integral_constant<int, 1>{});
     direction(std::integral_constant<int, 2>{});
+    {
+        int f0, f1, f2;
+        dims(2, f0, f1, f2);
+        for (int t = threadIdx.x; t < C::NPAIR * ncell; t += C::NT)
+            sip_face_add<K, Q, MODE, 2>(a, G, rows, R, ncell, b1, b2, f1, f2, t);
+    }
     __syncthreads();
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
