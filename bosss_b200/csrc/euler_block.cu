@@ -45,10 +45,7 @@ ModalTile euler_tiling(const EvalArgs& a) {
                 for (int f : fd)
                     cta += 3.9 * rounds(f * C::Q * C::Q, C::NT) + 2.5 * rounds(C::NROW * f + 5 * cells, C::NT) +
                            1.0 * rounds(C::NOUT * f, C::NT);
-                // fewer CTAs than SMs run alone on theirs, up to MINB share one
-                const double sm = tiles / 148.0;
-                const double share = 0.6 + 0.4 * (sm - 1.0) / std::max(1, C::MINB - 1);
-                const double waves = sm <= 1.0 ? 0.6 : sm <= C::MINB ? share : sm / C::MINB;
+                const double waves = tile_waves(tiles, C::MINB);
                 const double cost = waves * cta;
                 if (cost < bc) {
                     bc = cost;

@@ -13,6 +13,8 @@ namespace {
 // phases of a block (staged cells, faces, volume), the faces between blocks being evaluated twice
 template <class C>
 ModalTile sip_tiling(const EvalArgs& a) {
+    // volume round against a face-row round: QV^2 nodes of a slab against Q of a row
+    const double VW = 0.6 * C::QV * C::QV / C::FQ;
     const GridConst& g = a.g;
     const bool rev = g.stride[0] == 1 && g.stride[2] != 1;
     const int n0 = rev ? g.n[2] : g.n[0], n1 = g.n[1], n2 = rev ? g.n[0] : g.n[2];
@@ -40,11 +42,13 @@ ModalTile sip_tiling(const EvalArgs& a) {
                 const int fmax = cells + std::max(b1 * b2, std::max(b0 * b2, b0 * b1));
                 if (cells > C::CELLS || (b0 + 2) * (b1 + 2) * (b2 + 2) > C::SLOTS || fmax > C::FACES) continue;
                 const long long t0 = (m0 + b0 - 1) / b0, t1 = (n1 + b1 - 1) / b1, t2 = (n2 + b2 - 1) / b2;
-                const double tiles = (double)t0 * t1 * t2, slots = 148.0 * C::MINB;
-                const double faces = 3.0 * cells + b1 * b2 + b0 * b2 + b0 * b1;
-                // a CTA's time: fixed part (staging latency, barriers) + its work over its threads
-                const double cta = 40.0 + cells * 1.0 + faces * 0.8;
-                const double waves = tiles <= slots ? 1.0 : tiles / slots;
+                const double tiles = (double)t0 * t1 * t2;
+                // a CTA's time from the rounds of its phases (weights: measured shares, k = 2 and 4)
+                auto rounds = [](int tasks) { return (double)((tasks + C::NT - 1) / C::NT); };
+                const int fd[3] = {cells + b1 * b2, cells + b0 * b2, cells + b0 * b1};
+                double cta = 2.0 + VW * rounds(cells * C::QV) + 0.6 * rounds(cells * C::NPAIR);
+                for (int f : fd) cta += 2.0 * rounds(f * C::FQ) + 0.8 * rounds(2 * C::NG * f + C::NPAIR * cells);
+                const double waves = tile_waves(tiles, C::MINB);
                 const double cost = waves * cta;
                 if (cost < bc) {
                     bc = cost;

@@ -27,7 +27,7 @@ namespace bosss {
 template <int K, int Q, int MODE>
 struct SipCfg {
     static constexpr int NP = np_of(3, K), NPAIR = (K + 1) * (K + 2) / 2;
-    static constexpr int QV = Q < 2 * K ? Q : 2 * K;
+    static constexpr int QV = Q < 2 * K ? Q : 2 * K, FQ = Q;
     static constexpr int NG = MODE == MODE_RES ? 1 : 2;
     static constexpr int S = NP | 1;
     // threads, largest block, its halo box and its faces per direction (swept on B200; k = 4 residual at

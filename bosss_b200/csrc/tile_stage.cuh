@@ -17,6 +17,17 @@ __device__ __forceinline__ void tile_cp_wait() {
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
 }
 
+// Time of `tiles` CTAs in units of one CTA's time in a full wave of 148 x per_sm: whole waves, and for
+// the rest the pace of an SM that holds fewer CTAs (a CTA alone on its SM runs at about 0.6 of its
+// time among three); many waves overlap and count by their share
+inline double tile_waves(double tiles, int per_sm) {
+    const double slots = 148.0 * per_sm, w = tiles / slots;
+    if (w >= 4.0) return w;
+    const double full = (double)(long long)w, sm = (tiles - full * slots) / 148.0;
+    const double rest = sm <= 0.0 ? 0.0 : sm <= 1.0 ? (per_sm == 1 ? 1.0 : 0.6) : 0.6 + 0.4 * (sm - 1.0) / (per_sm - 1);
+    return full + rest;
+}
+
 // memory-order view of a three-dimensional grid and the block of one tile
 struct TileGeom {
     bool rev;          // GlobalID order: x fastest
