@@ -3,6 +3,7 @@
 #include <algorithm>
 
 #include "modal_kernel.cuh"
+#include "tile_stage.cuh"
 
 namespace bosss {
 
@@ -75,21 +76,20 @@ ModalTile modal_tiling(const EvalArgs& a, int D, int K, bool shared) {
     const long long plane = (long long)n1 * n2;
     const int s0 = (int)(a.cbeg / plane), s1 = (int)std::min<long long>(n0, (a.cend + plane - 1) / plane);
     const int m0 = std::max(1, s1 - s0);
-    (void)K;
+    const int per_sm = D == 2 || K <= 1 ? 4 : K == 2 ? 4 : K == 3 ? 2 : 1;
     // the extents depend on the sizes alone: the last ones found on this thread are kept, since
     // the search (a few hundred candidates) costs as much as a launch
     struct Memo {
-        int D = 0, m0 = 0, n1 = 0, n2 = 0, shared = 0;
+        int D = 0, K = 0, m0 = 0, n1 = 0, n2 = 0, shared = 0;
         ModalTile t{};
     };
     static thread_local Memo memo;
-    if (memo.D == D && memo.m0 == m0 && memo.n1 == n1 && memo.n2 == n2 && memo.shared == (int)shared) {
+    if (memo.D == D && memo.m0 == m0 && memo.n1 == n1 && memo.n2 == n2 && memo.shared == (int)shared && memo.K == K) {
         ModalTile t = memo.t;
         t.s0 = s0;
         return t;
     }
-    // extents within the halo box of the slots; the cost of a tile is its staged cells plus a fixed
-    // part (launch, latency), and CTAs run in waves of about 2 per SM
+    // extents within the halo box of the slots
     ModalTile best{};
     double bc = 1e300;
     const int c0[] = {1, 2, 3, 4, 5, 6, 8}, c2[] = {2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 16};
@@ -103,8 +103,9 @@ ModalTile modal_tiling(const EvalArgs& a, int D, int K, bool shared) {
                 const long long t0 = (m0 + b0 - 1) / b0, t1 = (n1 + b1 - 1) / b1, t2 = (n2 + b2 - 1) / b2;
                 const double tiles = (double)t0 * t1 * t2;
                 const double staged = (double)b0 * b1 * b2 + 2.0 * b1 * b2 + 2.0 * b0 * b1 + (D == 3 ? 2.0 * b0 * b2 : 0.0);
-                const double waves = shared ? tiles : std::max(1.0, tiles / (148.0 * 2));
-                const double cost = waves * (staged + 128.0 + 60.0);
+                // a CTA's time: fixed latencies (tile, runs, barriers), its copies and its cells (measured cycles)
+                const double cta = 7.0 + 0.016 * staged + 0.02 * b0 * b1 * b2;
+                const double cost = (shared ? tiles : tile_waves(tiles, per_sm)) * cta;
                 if (cost < bc) {
                     bc = cost;
                     best.b[0] = b0;
@@ -117,6 +118,7 @@ ModalTile modal_tiling(const EvalArgs& a, int D, int K, bool shared) {
             }
     best.ncell = best.b[0] * best.b[1] * best.b[2];
     memo.D = D;
+    memo.K = K;
     memo.m0 = m0;
     memo.n1 = n1;
     memo.n2 = n2;
