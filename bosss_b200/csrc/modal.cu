@@ -38,7 +38,7 @@ cudaError_t launch_modal(const EvalArgs& a, cudaStream_t s) {
 
 template <int D, int K, bool SIP>
 KernelEntry entry_of(int mode) {
-    KernelEntry e{nullptr, MODAL_CELLS, ModalCfg<D, K>::SMEM};
+    KernelEntry e{nullptr, ModalCfg<D, K>::CELLS, ModalCfg<D, K>::SMEM};
     e.launch = mode == MODE_RES   ? &launch_modal<D, K, SIP, MODE_RES>
                : mode == MODE_JVP ? &launch_modal<D, K, SIP, MODE_JVP>
                                   : &launch_modal<D, K, SIP, MODE_VJP>;
@@ -76,7 +76,25 @@ ModalTile modal_tiling(const EvalArgs& a, int D, int K, bool shared) {
     const long long plane = (long long)n1 * n2;
     const int s0 = (int)(a.cbeg / plane), s1 = (int)std::min<long long>(n0, (a.cend + plane - 1) / plane);
     const int m0 = std::max(1, s1 - s0);
-    const int per_sm = D == 2 || K <= 1 ? 4 : K == 2 ? 4 : K == 3 ? 2 : 1;
+    int cells = 0, box = 0, per_sm = 1;
+    auto cfg = [&](auto c) {
+        using C = decltype(c);
+        cells = C::CELLS;
+        box = C::BOX;
+        per_sm = std::min(C::MINB, 4);
+    };
+    switch (D * 10 + K) {
+        case 20: cfg(ModalCfg<2, 0>{}); break;
+        case 21: cfg(ModalCfg<2, 1>{}); break;
+        case 22: cfg(ModalCfg<2, 2>{}); break;
+        case 23: cfg(ModalCfg<2, 3>{}); break;
+        case 24: cfg(ModalCfg<2, 4>{}); break;
+        case 30: cfg(ModalCfg<3, 0>{}); break;
+        case 31: cfg(ModalCfg<3, 1>{}); break;
+        case 32: cfg(ModalCfg<3, 2>{}); break;
+        case 33: cfg(ModalCfg<3, 3>{}); break;
+        default: cfg(ModalCfg<3, 4>{}); break;
+    }
     // the extents depend on the sizes alone: the last ones found on this thread are kept, since
     // the search (a few hundred candidates) costs as much as a launch
     struct Memo {
@@ -97,9 +115,7 @@ ModalTile modal_tiling(const EvalArgs& a, int D, int K, bool shared) {
         for (int b1 : c0)
             for (int b2 : c2) {
                 if (D == 2 && b1 != 1) continue;
-                if (b0 * b1 * b2 > MODAL_CELLS) continue;
-                if (D == 3 && (b0 + 2) * (b1 + 2) * (b2 + 2) > 6 * 6 * 10) continue;
-                if (D == 2 && (b0 + 2) * (b2 + 2) > 10 * 18) continue;
+                if (b0 * b1 * b2 > cells || (b0 + 2) * (D == 3 ? b1 + 2 : 1) * (b2 + 2) > box) continue;
                 const long long t0 = (m0 + b0 - 1) / b0, t1 = (n1 + b1 - 1) / b1, t2 = (n2 + b2 - 1) / b2;
                 const double tiles = (double)t0 * t1 * t2;
                 const double staged = (double)b0 * b1 * b2 + 2.0 * b1 * b2 + 2.0 * b0 * b1 + (D == 3 ? 2.0 * b0 * b2 : 0.0);

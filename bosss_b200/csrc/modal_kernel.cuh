@@ -34,8 +34,6 @@
 namespace bosss {
 
 
-static constexpr int MODAL_CELLS = 128;   // cells of the largest tile
-
 template <int D, int K>
 struct ModalCfg {
     static constexpr int NP = np_of(D, K);
@@ -43,17 +41,19 @@ struct ModalCfg {
     static constexpr int PENCILS = D == 3 ? (K + 1) * (K + 2) / 2 : K + 1;
     // threads per cell: the pencils of a direction are dealt to T threads
     static constexpr int T = D == 2 ? 1 : (K == 4 ? 4 : K == 3 ? 2 : 1);
-    static constexpr int MINB = D == 2 ? 4 : (K == 4 ? 1 : K == 3 ? 2 : K == 2 ? 4 : 8);
-    static constexpr int NT = MODAL_CELLS * T;
+    static constexpr int MINB = D == 2 ? 4 : (K >= 3 ? 2 : K == 2 ? 4 : 8);
+    // cells of the largest tile and its halo box: 4 x 4 x 8 or 4 x 4 x 4 cells in 3D, 8 x 16 in 2D
+    static constexpr int CELLS = D == 3 && K == 4 ? 64 : 128;
+    static constexpr int BOX = D == 2 ? 10 * 18 : CELLS == 64 ? 6 * 6 * 6 : 6 * 6 * 10;
+    static constexpr int NT = CELLS * T;
     // runs a warp copies at a time: few warps have several each (k = 2, 48^3: 29 -> 23 us), sixteen warps
     // one or two (k = 4: four at a time 59 -> 71 us)
     static constexpr int GRP = T == 1 ? 4 : T == 2 ? 2 : 1;
-    // halo box of the largest tile: 4 x 4 x 8 cells in 3D, 8 x 16 in 2D, one zero slot, the results
-    static constexpr int SLOTS = (D == 3 ? 6 * 6 * 10 : 10 * 18) + 1;
+    static constexpr int SLOTS = BOX + 1;   // and one zero slot
     // runs of cells to copy: per row of the tile its cells (with the halo cells that follow on), and
     // halo cells across a periodic wrap; the rows of the slow and middle halos
     static constexpr int ROWS = D == 3 ? 128 : 16, RUNS = 3 * ROWS;
-    static constexpr size_t SMEM = sizeof(double) * (S * (SLOTS + MODAL_CELLS) + 3 * 2 * 6);
+    static constexpr size_t SMEM = sizeof(double) * (S * (SLOTS + CELLS) + 3 * 2 * 6);
 };
 struct ModalRun {
     long long src;   // first double
@@ -340,7 +340,7 @@ __device__ __forceinline__ void modal_tile(const EvalArgs& a, const Tables1D& T,
     };
     double* zero = sm + (C::SLOTS - 1) * S;
     double* res = sm + C::SLOTS * S;
-    double* fct = res + MODAL_CELLS * S;   // [direction][side]: coefficients of a face between plain cells
+    double* fct = res + C::CELLS * S;   // [direction][side]: coefficients of a face between plain cells
     if (tid < NP) zero[tid] = 0.0;
 
     // ---- stage the tile and its face halo: the runs of consecutive cells are found by one thread each
@@ -412,7 +412,7 @@ __device__ __forceinline__ void modal_tile(const EvalArgs& a, const Tables1D& T,
     asm volatile("cp.async.commit_group;\n" ::: "memory");
 
     // ---- the thread's cell and share of the pencils
-    const int cell = tid % MODAL_CELLS, th = tid / MODAL_CELLS;   // th is warp-uniform
+    const int cell = tid % C::CELLS, th = tid / C::CELLS;   // th is warp-uniform
     const int l0 = cell / (b1 * b2), lr = cell - l0 * b1 * b2;
     const int l1 = lr / b2, l2 = lr - l1 * b2;
     const int c0 = o0 + l0, c1 = o1 + l1, c2 = o2 + l2;
