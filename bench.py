@@ -984,9 +984,9 @@ def main():
     # ncu figures per call (summed over the call's launches) exist for the 32^3 k=3 workload
     # on the slab path ("euler3d_*") and on the face-once path ("euler3d_faces_*")
     def _prof(table, path, what):
-        if (args.n, args.k) != (32, 3) or path not in (2, 3):
+        if (args.n, args.k) != (32, 3) or path not in (2, 3, 7):
             return None
-        return table.get(("euler3d_" if path == 2 else "euler3d_faces_") + what)
+        return table.get({2: "euler3d_", 3: "euler3d_faces_", 7: "euler3d_blocks_"}[path] + what)
     per_kernel = {
         "residual": {"ms": t_r * 1e3, "algorithmic_bytes": bytes_res, "hbm_gbs": bytes_res / t_r / 1e9,
                      "launches": launch_res, "kernels": PATH_KERNELS[path_res] % "RESIDUAL",
