@@ -9,16 +9,17 @@
 //            thread per face side; SIP reads no tangential derivative), one thread per (face, node
 //            row) for the forms, then (cell, pencil) threads contract the rows and add both faces
 //            of a cell. Faces between two blocks are evaluated by both.
-// Bound by the FP64 pipe: the quadrature nodes of nu(u) (Q = 2K+1 for order 4K) carry 10-100x the
-// arithmetic of the modes.
+// The quadrature nodes of nu(u) (Q = 2K+1 for order 4K) carry 10-100x the arithmetic of the modes.
+// At 48^3 k = 2 the FP64 pipe is 41 % busy and 52 % of the issue slots are used; the rest are the
+// latencies between the phases of a block.
 //
 // Volume nodes: with nu a quadratic of u the volume integrand nu grad u . grad v has total degree
 // 4K - 2, so the Gauss rule with 2K nodes per direction (exact to degree 4K - 1) gives the same
 // integrals as any larger one; the volume uses min(Q, 2K) nodes (K = 2, Q = 5: 64 instead of 125).
 // The faces keep Q: the penalty term reaches degree 4K and takes a maximum of two viscosities.
 //
-// Measured on B200 against the slab / generic tiles: J v at 48^3 k = 2 (Q = 5) 1.40 -> 0.216 ms,
-// residual + J^T w at 21x16x18 k = 4 (Q = 9) 1.13 -> 0.245 ms.
+// Measured on B200 against the slab / generic tiles: J v at 48^3 k = 2 (Q = 5) 1.40 -> 0.210 ms,
+// residual + J^T w at 21x16x18 k = 4 (Q = 9) 1.14 -> 0.226 ms.
 #pragma once
 #include "tile_stage.cuh"
 

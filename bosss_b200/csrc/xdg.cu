@@ -502,7 +502,7 @@ __device__ __forceinline__ double warp_sums(double (&v)[32]) {
 // The item's contributions go to its slot of item_out (own cell, then the face neighbour), which
 // k_cut_gather adds into the cells in a fixed order -- no atomics, so the result is the same bits
 // run to run. Latency-bound: items have 8 to 125 nodes; the first version (64 threads per item,
-// full gradients, 2 NP block reductions of 5 steps) took 115 us per species at 80^3, k = 2.
+// full gradients, 2 NP block reductions of 5 steps) took 115 us per species at 80^3, k = 2, this one 47 us.
 template <int K>
 __global__ void __launch_bounds__(128) k_cut_eval(const CutItem* __restrict__ items, int nitems, const double* __restrict__ nodes,
                                                   const double* __restrict__ weights, EvalArgs a, double* __restrict__ item_out) {
@@ -1659,7 +1659,7 @@ int bosss_b200_xdg_create(const bosss_op_desc* opA, const bosss_op_desc* opB, co
         xo.rule = xopt->rule;
     }
     if (xo.rule != 0 && xo.rule != 1) return fail(BOSSS_ERR_BAD_ARG, "XDG rule family: 0 or 1");
-    // the species masks of the bulk evaluation are read by the generic and the slab kernels
+    // the species masks of the bulk evaluation are read by the modal, the generic and the slab kernels
     bosss_options hopt{};
     if (opt) hopt = *opt;
     if (hopt.kernel == 3) return fail(BOSSS_ERR_BAD_ARG, "XDG evaluation: kernel 0, 1 or 2");
@@ -1933,7 +1933,7 @@ int bosss_b200_xdg_evaluate_device(bosss_xdg* X, int32_t species, double alpha, 
             if (rc) return rc;
         }
     }
-    // cut cells and faces: explicit rules, added atomically
+    // cut cells and faces: explicit rules; each item fills its slot, k_cut_gather adds the slots in a fixed order
     const int n = (int)X->items[s].size();
     if (n > 0) {
         EvalArgs a = h->base;
