@@ -435,6 +435,8 @@ __device__ __forceinline__ void modal_tile(const EvalArgs& a, const Tables1D& T,
     const double* own = sm + (active ? slot(l0, l1, l2) : 0);
     // a cell without any standard term takes no part (its coefficients may be anything)
     if (MASK && volm == 0.0 && fmask == 0) own = zero;
+    const bool transport = a.ph.has_transport != 0, diffusion = SIP && a.ph.has_sip != 0;
+    if (MODE != MODE_VJP && !transport && !diffusion) own = zero;   // a source alone reads no coefficients
     double* R = res + cell * S;
     // a face between two cells away from the boundaries of the global grid has the same
     // coefficients everywhere (unless the caller gives length scales): computed once per CTA
@@ -474,10 +476,13 @@ __device__ __forceinline__ void modal_tile(const EvalArgs& a, const Tables1D& T,
                     fc[s] = modal_face<D, SIP, MODE>(a, ijk, DIR, s, on, h[s]);
                 }
             }
-            const bool hl = h[0], hu = h[1];
             const FaceCoef &fl = fc[0], &fu = fc[1];
-            const double* nbu = hu ? own + sl : zero;
-            const double* nbl = hl ? own - sl : zero;
+            // a neighbour is read only where the form reads it, with diffusion everywhere, else where the
+            // upwind flux takes its value: a zero coefficient times a NaN or Inf would carry it
+            // upwind (J^T w takes the jump of w on both sides, as the quadrature kernels do)
+            const bool every = MODE == MODE_VJP || diffusion, low = vel > 0.0;   // low: the flux takes the lower cell's value
+            const double* nbu = h[1] && (every || (transport && !low)) ? own + sl : zero;
+            const double* nbl = h[0] && (every || (transport && low)) ? own - sl : zero;
             const double vT = -2.0 * vel * thd * volm, vS = -2.0 * nu0 * thd * thd * volm;
             if constexpr (C::T == 1) {
                 modal_pencils<D, K, SIP, MODE, DIR, 0>(T, own, nbu, nbl, fu, fl, vT, vS, R);
