@@ -917,6 +917,10 @@ static int host_pipelined(bosss_handle* h, const HostJob* jobs, int njobs, const
     if (h->check_nan)
         for (int k = 0; k < njobs; ++k) {
             rc = check_nan(h, jobs[k].dY, nY(jobs[k]) * J, s);
+            // the quadrature kernels form nu(u) in both products, also where nu2 = 0, so that a NaN or Inf
+            // of the state shows in the output; the modal kernel does not read the state there
+            if (!rc && jobs[k].mode != MODE_RES && h->kern_variant[jobs[k].mode] == VARIANT_MODAL && h->base.ph.has_sip)
+                rc = check_nan(h, h->dU, h->ndom, s);
             if (rc) return finish(rc);
         }
     e = cudaStreamSynchronize(so);

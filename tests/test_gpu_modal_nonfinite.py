@@ -55,3 +55,22 @@ def test_nonfinite_values_reach_the_same_cells(n, periodic, kind, value):
                 ev.Evaluate(1.0, 0.0, out, v)
                 sets.append([bad_cells(t, cells) for t in (out, ev.jvp(u, v), ev.vjp(u, v))])
         assert sets[0] == sets[1], (k, sets)
+
+
+@pytest.mark.parametrize("kernel", [C.KERNEL_AUTO, C.KERNEL_GENERIC], ids=["modal", "generic"])
+def test_nan_check_refuses_products_at_a_nonfinite_state(kernel):
+    """With the NaN check on, J v and J^T w of a diffusion operator at a state with a NaN or Inf are
+    refused, on the modal kernel too, which does not read the state for them."""
+    n, k = (3, 4, 2), 2
+    op, g, dom, cod = make(n, k, COMPS["advdiff"](3), (True, False, True))
+    U = np.random.default_rng(1).uniform(-1, 1, g.NoOfCells * dom[0].Np)
+    with op.GetEvaluatorEx(dom, None, cod, kernel=kernel, check_nan=True) as ev:
+        ev.jvp(U, U)
+        ev.vjp(U, U)
+        for value in (np.nan, np.inf):
+            bad = U.copy()
+            bad[77] = value
+            for product in (ev.jvp, ev.vjp):
+                with pytest.raises(C.BosssError) as e:
+                    product(bad, U)
+                assert e.value.code == C.ERR_NAN
