@@ -65,13 +65,14 @@ __device__ __forceinline__ constexpr int eul_mode(int m, int p, int r) {
 }
 
 // HLLC flux through a face normal to the first momentum component (the caller permutes), as
-// PhysEuler::inner. Divisions by two state-dependent values share one reciprocal of the product
+// PhysEuler::inner. The divisions by the two wave-speed differences share one reciprocal of their product;
+// the densities have one each: their product leaves the double range where the densities do not,
+// and a NaN or zero density of one side would reach the flux of the other
 template <class T>
 __device__ __forceinline__ void hllc_flux(const PhysParams& p, const T* UA, const T* UB, T* f) {
     const double MS = p.gamma * p.mach * p.mach, G2 = 0.5 * (p.gamma + 1.0) / p.gamma, gm1 = p.gamma - 1.0;
     constexpr int N = 0;
-    const T irAB = 1.0 / (UA[0] * UB[0]);
-    const T irA = UB[0] * irAB, irB = UA[0] * irAB;
+    const T irA = 1.0 / UA[0], irB = 1.0 / UB[0];
     const T unA = UA[1 + N] * irA, unB = UB[1 + N] * irB;
     const T kA = (UA[1] * UA[1] + UA[2] * UA[2] + UA[3] * UA[3]) * irA;
     const T kB = (UB[1] * UB[1] + UB[2] * UB[2] + UB[3] * UB[3]) * irB;
@@ -114,8 +115,7 @@ __device__ __forceinline__ void hllc_adj(const PhysParams& p, const double* UA, 
                                          double* UAb, double* UBb) {
     const double g = p.gamma, gm1 = g - 1.0, MS = g * p.mach * p.mach, iMS = p.ims, G2 = 0.5 * (g + 1.0) / g;
     constexpr int N = 0;
-    const double rA = UA[0], rB = UB[0], irAB = 1.0 / (rA * rB);
-    const double irA = rB * irAB, irB = rA * irAB;
+    const double rA = UA[0], rB = UB[0], irA = 1.0 / rA, irB = 1.0 / rB;
     const double unA = UA[1 + N] * irA, unB = UB[1 + N] * irB;
     const double kA = (UA[1] * UA[1] + UA[2] * UA[2] + UA[3] * UA[3]) * irA;
     const double kB = (UB[1] * UB[1] + UB[2] * UB[2] + UB[3] * UB[3]) * irB;

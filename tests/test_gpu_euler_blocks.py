@@ -83,3 +83,51 @@ def test_euler_blocks_cell_ranges():
                 want = torch.full_like(u, 9.0)
                 want[lo * npc:hi * npc] = whole[lo * npc:hi * npc]
                 assert torch.equal(c, want), (mode, lo, hi)
+
+
+@pytest.mark.parametrize("speed", [0.1, 3.0], ids=["subsonic", "supersonic"])
+@pytest.mark.parametrize("k", [1, 3])
+def test_densities_whose_product_leaves_the_double_range(k, speed):
+    """rho -> A rho, u -> B u, p -> A B^2 p is an exact symmetry; with powers of two every operation of
+    the kernels scales exactly, so all three products give the scaled bits."""
+    import torch
+    op, g, dom, cod, U = make((3, 4, 5), k, C.CELLS_GENERATOR, 11 + k, speed)
+    J, A, B = g.NoOfCells, 2.0 ** 515, 2.0 ** -10      # rho_A rho_B about 2^1030, momentum^2 below 2^1016
+    su = np.array([A, A * B, A * B, A * B, A * B * B])[None, :, None]
+    sf = su * B
+    U = U.reshape(J, 5, -1)
+    r = np.random.default_rng(k)
+    V, W = r.uniform(-1, 1, U.shape), r.uniform(-1, 1, U.shape)
+    res = []
+    with op.GetEvaluatorEx(dom, None, cod) as ev:
+        for s, f in ((1.0, 1.0), (su, sf)):
+            u, v, w = (torch.from_numpy(np.ascontiguousarray(t).ravel()).cuda() for t in (U * s, V * s, W / f))
+            out = torch.zeros_like(u)
+            ev.Evaluate(1.0, 0.0, out, u)
+            res.append([t.cpu().numpy().reshape(U.shape) for t in (out, ev.jvp(u, v), ev.vjp(u, w))])
+    for a, b, s in zip(res[0], res[1], (sf, sf, 1.0 / su)):
+        assert np.isfinite(a).all() and np.array_equal(a * s, b)
+
+
+@pytest.mark.parametrize("value", [np.nan, 0.0], ids=["nan", "vacuum"])
+@pytest.mark.parametrize("speed", [0.1, 3.0], ids=["subsonic", "supersonic"])
+def test_a_bad_density_reaches_the_cells_it_reaches_on_the_slab_kernel(speed, value):
+    """The flux reads the upwind state only where the waves run one way: a NaN or vanishing density of a
+    cell reaches the same cells as on the quadrature slab kernel."""
+    import torch
+    k = 2
+    op, g, dom, cod, U = make((5, 4, 6), k, C.CELLS_GENERATOR, 3, speed)
+    J = g.NoOfCells
+    V = np.random.default_rng(5).uniform(-1, 1, U.size)
+    U = U.reshape(J, 5, -1)
+    U[J // 2, 0, :] = 0.0
+    U[J // 2, 0, 0] = value
+    u, v = torch.from_numpy(U.ravel()).cuda(), torch.from_numpy(V).cuda()
+    sets = []
+    for kernel in (C.KERNEL_AUTO, C.KERNEL_SLAB):
+        with op.GetEvaluatorEx(dom, None, cod, kernel=kernel) as ev:
+            out = torch.zeros_like(u)
+            ev.Evaluate(1.0, 0.0, out, u)
+            sets.append([np.nonzero(~np.isfinite(t.cpu().numpy().reshape(J, -1)).all(axis=1))[0].tolist()
+                         for t in (out, ev.jvp(u, v), ev.vjp(u, v))])
+    assert sets[0] == sets[1]
