@@ -238,21 +238,27 @@ __device__ __forceinline__ void modal_pencils(const Tables1D& T, const double* o
             }
             const double gs = gu + gl, gd = gu - gl;
             // volume: int L_a' L_m = 2 L_a(1) L_m(1) (m < a, a - m odd), int L_a' L_m' = 2 c_min L_a(1) L_m(1)
-            // (a - m even): sums over the modes below / above by parity
-            double pre[2] = {0.0, 0.0}, pc[2] = {0.0, 0.0}, up[2] = {ue, uo};
+            // (a - m even): sums over the modes below / above by parity. above[m]: mode m and those above it of
+            // its parity, added directly (what is left of the total after the modes below would carry
+            // their rounding: a large mean beside small variations)
+            double pre[2] = {0.0, 0.0}, pc[2] = {0.0, 0.0}, above[L1 + 2];
+#pragma unroll
+            for (int m = L1 + 1; m >= 0; --m) above[m] = 0.0;
+#pragma unroll
+            for (int m = L1 - 1; m >= 0; --m)
+                if (m < L) above[m] = w[m] + above[m + 2];
 #pragma unroll
             for (int m = 0; m < L1; ++m)
                 if (m < L) {
                     const int n = pencil_mode<D>(DIR, m, p, r);
                     const double c = 0.5 * m * (m + 1);
                     const int e = m & 1;
-                    up[e] -= w[m];   // modes above m of the same parity
                     double h = e ? gd : gs;
-                    if (MODE == MODE_VJP) h += vT * up[1 - e];   // the other parity: those above m are left
+                    if (MODE == MODE_VJP) h += vT * above[m + 1];
                     else h += vT * pre[1 - e];
                     if (SIP && m > 0) {
                         pc[e] += c * w[m];
-                        h += vS * pc[e] + c * ((e ? Gs : Gd) + vS * up[e]);
+                        h += vS * pc[e] + c * ((e ? Gs : Gd) + vS * above[m + 2]);
                     }
                     pre[e] += w[m];
                     if (DIR == 0) R[n] = h * T.e[1][m];

@@ -99,3 +99,35 @@ def test_nonlinear_forms_keep_the_quadrature_kernels():
                                quad=O.QuadOrderFunc.NonLinear(3))
         with op.GetEvaluatorEx(dom, None, cod) as ev:
             assert (ev.kernel_info(0)[0] == 5) == (nu2 == 0.0)
+
+
+@pytest.mark.parametrize("n", [(2, 1, 3), (3, 2)], ids=["3d", "2d"])
+@pytest.mark.parametrize("kind", ["diffusion", "transport"])
+def test_modal_volume_terms_of_small_variations_on_a_large_mean(n, kind):
+    """Equal cells with even modes only: the jumps vanish exactly and the derivatives do not see the
+    mean, so products of a field 2^40 + O(1) are accurate relative to the O(1) part."""
+    import torch
+    dim = len(n)
+    for k in (2, 3, 4):
+        comp = O.SIPLaplace(4.0, "u", nu0=0.3) if kind == "diffusion" else O.ScalarTransportFlux([0.7, -0.4, 0.3][:dim], "u")
+        op, g, dom, cod = make(n, k, [comp], (True,) * dim)
+        desc = (op.descriptor([k], [k], dim), g.desc())
+        # modes by total degree, then the first exponents
+        exps = [e for d in range(k + 1) for e in np.ndindex(*(k + 1,) * dim) if sum(e) == d]
+        r = np.random.default_rng(k)
+        c = np.array([0.0 if any(i & 1 for i in e) else r.uniform(0.5, 1.0) for e in exps])
+        c[0] += 2.0 ** 40
+        U = np.tile(c, g.NoOfCells)
+        u = torch.from_numpy(U).cuda()
+        with op.GetEvaluatorEx(dom, None, cod) as ev:
+            assert ev.kernel_info(0)[0] == 5
+            if kind == "transport":
+                pairs = [(ev.vjp(u, u), orc.vjp(*desc, U, U))]
+            else:     # a symmetric operator: J^T w = J w
+                out = torch.zeros_like(u)
+                ev.Evaluate(1.0, 0.0, out, u)
+                jvp = orc.jvp(*desc, U, U)
+                pairs = [(out, orc.evaluate(*desc, U)), (ev.jvp(u, u), jvp), (ev.vjp(u, u), jvp)]
+            for got, want in pairs:
+                assert np.linalg.norm(want) < 1e4     # the mean does not enter
+                assert rel(got.cpu().numpy(), want) <= TOL, k
