@@ -107,12 +107,15 @@ int bosss_b200_rk_steps_device(bosss_handle* h, int32_t stages, const double* a,
     if (rc) return rc;
     CUDA_TRY(cudaSetDevice(h->device));
     cudaStream_t st = stream ? (cudaStream_t)stream : h->stream;
-    // a graph costs its capture and instantiation (about 0.1 ms for four stages) once per call: it pays
-    // from GRAPH_STEPS steps on; below, the launches of a step (about 3 us each) run ahead of their
-    // kernels just as well (3 RK4 steps, 17x12x9 cells, k = 2: 269 us with a graph, 259 us without, of
-    // them 258 us in kernels).
-    constexpr int GRAPH_STEPS = 16;
-    if (!use_graph || nsteps < GRAPH_STEPS) {
+    // a graph costs about 0.24 ms of host time per call (capture, instantiation), plain launches about 4.1 us
+    // each, of which a small grid's kernels cover a half or less: about 60 launches break even. Measured
+    // (us per call, calls back to back, graph / plain): RK4 on 16^2 cells k = 2, 4 steps 266 / 133, 8 steps
+    // (64 launches) 271 / 264, 15 steps 325 / 494; Euler 4^3 k = 1, 4 steps 270 / 265, 8 steps 429 / 527; Heun on
+    // 16^2, 16 steps (64) 277 / 395; explicit Euler on 4^3, 16 steps (32) 325 / 267, 32 steps (64) 479 / 530.
+    // Where the kernels cover the launches (17x12x9 k = 2, 3 steps: 269 / 259) only the 0.01 ms of
+    // the capture that they do not cover is at stake
+    constexpr long long GRAPH_LAUNCHES = 64;
+    if (!use_graph || 2LL * stages * nsteps < GRAPH_LAUNCHES) {
         for (int i = 0; i < nsteps; ++i) {
             rc = rk_step(h, T, dt, time + i * dt, U_dev, work_dev, st);
             if (rc) return rc;

@@ -169,7 +169,8 @@ class RungeKutta:
         return dt
 
     def PerformDevice(self, U, dt, nsteps=1, use_graph=True):
-        """Advance the CUDA tensor ``U`` in place (enqueued on the current torch stream)."""
+        """Advance the CUDA tensor ``U`` in place (enqueued on the current torch stream).
+        ``use_graph``: calls of 64 kernel launches or more replay a captured step (same bits)."""
         import torch
         n = self.work_size()
         if self._work is None or self._work.numel() < n or self._work.device != U.device:

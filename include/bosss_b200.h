@@ -518,13 +518,14 @@ int bosss_b200_xdg_interface_evaluate_device(bosss_xdg* X, double alpha, const d
  * the caller; the Python mirror carries them. */
 int bosss_b200_rk_work_size(const bosss_handle* h, int32_t stages, int64_t* n_doubles);
 /* nsteps steps on device buffers: U_dev in/out, work_dev of bosss_b200_rk_work_size doubles.
- * use_graph != 0: one step is captured into a CUDA graph once and the graph is launched nsteps
- * times (one residual launch and one stage-combination launch per stage). Asynchronous on
- * `stream` (NULL: the handle's stream). */
+ * A step is one residual launch and one stage-combination launch per stage. use_graph != 0: calls
+ * of 64 launches or more (2 * stages * nsteps) capture one step into a CUDA graph and launch the
+ * graph nsteps times; shorter calls, where the capture would cost more than it saves, launch the
+ * kernels directly, with the same bits. Asynchronous on `stream` (NULL: the handle's stream). */
 int bosss_b200_rk_steps_device(bosss_handle* h, int32_t stages, const double* a, const double* b, const double* c,
                                double dt, int32_t nsteps, double time, double* U_dev, double* work_dev,
                                int32_t use_graph, void* stream);
-/* Same with a host state vector U (copied in, stepped with a captured graph, copied back). */
+/* Same with a host state vector U (copied in, stepped as with use_graph = 1, copied back). */
 int bosss_b200_rk_steps(bosss_handle* h, int32_t stages, const double* a, const double* b, const double* c, double dt,
                         int32_t nsteps, double time, double* U);
 

@@ -185,3 +185,22 @@ def test_rk_captured_step_equals_plain_launches():
         T.RungeKutta(s, ev, None).PerformDevice(Up, 1e-3, nsteps=17, use_graph=False)
         torch.cuda.synchronize()
         assert torch.equal(Ug, Up)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,nsteps", [("RungeKutta1901", 7), ("RungeKutta1901", 8), ("Heun", 15), ("Heun", 16),
+                                         ("RungeKutta1901", 15), ("RungeKutta1901", 16)])
+def test_rk_on_both_sides_of_the_capture_rule(name, nsteps):
+    """Calls just below 64 launches (plain) and from there on (a captured step replayed): the bits of
+    plain launches, and the oracle's steps."""
+    import torch
+    pr = P.euler3d(n=4, k=3, seed=41)
+    s = getattr(T.RungeKuttaScheme, name)()
+    with pr.evaluator() as ev:
+        Ug, Up = (torch.from_numpy(pr.U.copy()).cuda() for _ in range(2))
+        T.RungeKutta(s, ev, None).PerformDevice(Ug, 1e-3, nsteps=nsteps, use_graph=True)
+        T.RungeKutta(s, ev, None).PerformDevice(Up, 1e-3, nsteps=nsteps, use_graph=False)
+        torch.cuda.synchronize()
+        assert torch.equal(Ug, Up)
+    ref = orc.rk_steps(*pr.descs(), pr.U, s.a, s.b, s.c, 1e-3, nsteps)
+    assert _rel(Ug.cpu().numpy(), ref) <= 1e-12
