@@ -17,53 +17,42 @@ ModalTile euler_tiling(const EvalArgs& a) {
     const long long plane = (long long)n1 * n2;
     const int s0 = (int)(a.cbeg / plane), s1 = (int)std::min<long long>(n0, (a.cend + plane - 1) / plane);
     const int m0 = std::max(1, s1 - s0);
-    // the extents depend on the sizes alone: the last ones found on this thread are kept
-    struct Memo {
-        int m0 = 0, n1 = 0, n2 = 0;
-        ModalTile t{};
-    };
-    static thread_local Memo memo;
-    if (memo.m0 == m0 && memo.n1 == n1 && memo.n2 == n2) {
-        ModalTile t = memo.t;
-        t.s0 = s0;
-        return t;
-    }
-    ModalTile best{};
-    double bc = 1e300;
-    for (int b0 = 1; b0 <= 8; ++b0)
-        for (int b1 = 1; b1 <= 8; ++b1)
-            for (int b2 = 1; b2 <= 8; ++b2) {
-                const int cells = b0 * b1 * b2;
-                const int fmax = cells + std::max(b1 * b2, std::max(b0 * b2, b0 * b1));
-                if (cells > C::CELLS || fmax > C::FACES) continue;
-                const long long t0 = (m0 + b0 - 1) / b0, t1 = (n1 + b1 - 1) / b1, t2 = (n2 + b2 - 1) / b2;
-                const double tiles = (double)t0 * t1 * t2;
-                // a CTA's time from the rounds of its phases (weights: measured cycles per round, k = 3)
-                auto rounds = [](int tasks, int per) { return (double)((tasks + per - 1) / per); };
-                const int fd[3] = {cells + b1 * b2, cells + b0 * b2, cells + b0 * b1};
-                double cta = 8.0 + 7.3 * rounds(cells, C::NW * C::CW);
-                for (int f : fd)
-                    cta += 3.9 * rounds(f * C::Q * C::Q, C::NT) + 2.5 * rounds(C::NROW * f + 5 * cells, C::NT) +
-                           1.0 * rounds(C::NOUT * f, C::NT);
-                const double waves = tile_waves(tiles, C::MINB);
-                const double cost = waves * cta;
-                if (cost < bc) {
-                    bc = cost;
-                    best.b[0] = b0;
-                    best.b[1] = b1;
-                    best.b[2] = b2;
-                    best.t[0] = (int)t0;
-                    best.t[1] = (int)t1;
-                    best.t[2] = (int)t2;
+    static thread_local TileMemo memo;
+    ModalTile t = memo.get({{0, 0, m0, n1, n2, 0}}, [&] {
+        ModalTile best{};
+        double bc = 1e300;
+        for (int b0 = 1; b0 <= 8; ++b0)
+            for (int b1 = 1; b1 <= 8; ++b1)
+                for (int b2 = 1; b2 <= 8; ++b2) {
+                    const int cells = b0 * b1 * b2;
+                    const int fmax = cells + std::max(b1 * b2, std::max(b0 * b2, b0 * b1));
+                    if (cells > C::CELLS || fmax > C::FACES) continue;
+                    const long long t0 = (m0 + b0 - 1) / b0, t1 = (n1 + b1 - 1) / b1, t2 = (n2 + b2 - 1) / b2;
+                    const double tiles = (double)t0 * t1 * t2;
+                    // a CTA's time from the rounds of its phases (weights: measured cycles per round, k = 3)
+                    auto rounds = [](int tasks, int per) { return (double)((tasks + per - 1) / per); };
+                    const int fd[3] = {cells + b1 * b2, cells + b0 * b2, cells + b0 * b1};
+                    double cta = 8.0 + 7.3 * rounds(cells, C::NW * C::CW);
+                    for (int f : fd)
+                        cta += 3.9 * rounds(f * C::Q * C::Q, C::NT) + 2.5 * rounds(C::NROW * f + 5 * cells, C::NT) +
+                               1.0 * rounds(C::NOUT * f, C::NT);
+                    const double waves = tile_waves(tiles, C::MINB);
+                    const double cost = waves * cta;
+                    if (cost < bc) {
+                        bc = cost;
+                        best.b[0] = b0;
+                        best.b[1] = b1;
+                        best.b[2] = b2;
+                        best.t[0] = (int)t0;
+                        best.t[1] = (int)t1;
+                        best.t[2] = (int)t2;
+                    }
                 }
-            }
-    best.ncell = best.b[0] * best.b[1] * best.b[2];
-    memo.m0 = m0;
-    memo.n1 = n1;
-    memo.n2 = n2;
-    memo.t = best;
-    best.s0 = s0;
-    return best;
+        best.ncell = best.b[0] * best.b[1] * best.b[2];
+        return best;
+    });
+    t.s0 = s0;
+    return t;
 }
 
 template <int K, int MODE>

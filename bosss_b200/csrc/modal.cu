@@ -95,53 +95,38 @@ ModalTile modal_tiling(const EvalArgs& a, int D, int K, bool shared) {
         case 33: cfg(ModalCfg<3, 3>{}); break;
         default: cfg(ModalCfg<3, 4>{}); break;
     }
-    // the extents depend on the sizes alone: the last ones found on this thread are kept, since
-    // the search (a few hundred candidates) costs as much as a launch
-    struct Memo {
-        int D = 0, K = 0, m0 = 0, n1 = 0, n2 = 0, shared = 0;
-        ModalTile t{};
-    };
-    static thread_local Memo memo;
-    if (memo.D == D && memo.m0 == m0 && memo.n1 == n1 && memo.n2 == n2 && memo.shared == (int)shared && memo.K == K) {
-        ModalTile t = memo.t;
-        t.s0 = s0;
-        return t;
-    }
-    // extents within the halo box of the slots
-    ModalTile best{};
-    double bc = 1e300;
-    const int c0[] = {1, 2, 3, 4, 5, 6, 8}, c2[] = {2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 16};
-    for (int b0 : c0)
-        for (int b1 : c0)
-            for (int b2 : c2) {
-                if (D == 2 && b1 != 1) continue;
-                if (b0 * b1 * b2 > cells || (b0 + 2) * (D == 3 ? b1 + 2 : 1) * (b2 + 2) > box) continue;
-                const long long t0 = (m0 + b0 - 1) / b0, t1 = (n1 + b1 - 1) / b1, t2 = (n2 + b2 - 1) / b2;
-                const double tiles = (double)t0 * t1 * t2;
-                const double staged = (double)b0 * b1 * b2 + 2.0 * b1 * b2 + 2.0 * b0 * b1 + (D == 3 ? 2.0 * b0 * b2 : 0.0);
-                // a CTA's time: fixed latencies (tile, runs, barriers), its copies and its cells (measured cycles)
-                const double cta = 7.0 + 0.016 * staged + 0.02 * b0 * b1 * b2;
-                const double cost = (shared ? tiles : tile_waves(tiles, per_sm)) * cta;
-                if (cost < bc) {
-                    bc = cost;
-                    best.b[0] = b0;
-                    best.b[1] = b1;
-                    best.b[2] = b2;
-                    best.t[0] = (int)t0;
-                    best.t[1] = (int)t1;
-                    best.t[2] = (int)t2;
+    static thread_local TileMemo memo;
+    ModalTile t = memo.get({{D, K, m0, n1, n2, (int)shared}}, [&] {
+        // extents within the halo box of the slots
+        ModalTile best{};
+        double bc = 1e300;
+        const int c0[] = {1, 2, 3, 4, 5, 6, 8}, c2[] = {2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 16};
+        for (int b0 : c0)
+            for (int b1 : c0)
+                for (int b2 : c2) {
+                    if (D == 2 && b1 != 1) continue;
+                    if (b0 * b1 * b2 > cells || (b0 + 2) * (D == 3 ? b1 + 2 : 1) * (b2 + 2) > box) continue;
+                    const long long t0 = (m0 + b0 - 1) / b0, t1 = (n1 + b1 - 1) / b1, t2 = (n2 + b2 - 1) / b2;
+                    const double tiles = (double)t0 * t1 * t2;
+                    const double staged = (double)b0 * b1 * b2 + 2.0 * b1 * b2 + 2.0 * b0 * b1 + (D == 3 ? 2.0 * b0 * b2 : 0.0);
+                    // a CTA's time: fixed latencies (tile, runs, barriers), its copies and its cells (measured cycles)
+                    const double cta = 7.0 + 0.016 * staged + 0.02 * b0 * b1 * b2;
+                    const double cost = (shared ? tiles : tile_waves(tiles, per_sm)) * cta;
+                    if (cost < bc) {
+                        bc = cost;
+                        best.b[0] = b0;
+                        best.b[1] = b1;
+                        best.b[2] = b2;
+                        best.t[0] = (int)t0;
+                        best.t[1] = (int)t1;
+                        best.t[2] = (int)t2;
+                    }
                 }
-            }
-    best.ncell = best.b[0] * best.b[1] * best.b[2];
-    memo.D = D;
-    memo.K = K;
-    memo.m0 = m0;
-    memo.n1 = n1;
-    memo.n2 = n2;
-    memo.shared = shared;
-    memo.t = best;
-    best.s0 = s0;
-    return best;
+        best.ncell = best.b[0] * best.b[1] * best.b[2];
+        return best;
+    });
+    t.s0 = s0;
+    return t;
 }
 
 }  // namespace bosss

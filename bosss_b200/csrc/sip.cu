@@ -21,52 +21,41 @@ ModalTile sip_tiling(const EvalArgs& a) {
     const long long plane = (long long)n1 * n2;
     const int s0 = (int)(a.cbeg / plane), s1 = (int)std::min<long long>(n0, (a.cend + plane - 1) / plane);
     const int m0 = std::max(1, s1 - s0);
-    // the extents depend on the sizes alone: the last ones found on this thread are kept
-    struct Memo {
-        int m0 = 0, n1 = 0, n2 = 0;
-        ModalTile t{};
-    };
-    static thread_local Memo memo;
-    if (memo.m0 == m0 && memo.n1 == n1 && memo.n2 == n2) {
-        ModalTile t = memo.t;
-        t.s0 = s0;
-        return t;
-    }
-    ModalTile best{};
-    double bc = 1e300;
-    const int ext[] = {1, 2, 3, 4, 5, 6, 8};
-    for (int b0 : ext)
-        for (int b1 : ext)
-            for (int b2 : ext) {
-                const int cells = b0 * b1 * b2;
-                const int fmax = cells + std::max(b1 * b2, std::max(b0 * b2, b0 * b1));
-                if (cells > C::CELLS || (b0 + 2) * (b1 + 2) * (b2 + 2) > C::SLOTS || fmax > C::FACES) continue;
-                const long long t0 = (m0 + b0 - 1) / b0, t1 = (n1 + b1 - 1) / b1, t2 = (n2 + b2 - 1) / b2;
-                const double tiles = (double)t0 * t1 * t2;
-                // a CTA's time from the rounds of its phases (weights: measured shares, k = 2 and 4)
-                auto rounds = [](int tasks) { return (double)((tasks + C::NT - 1) / C::NT); };
-                const int fd[3] = {cells + b1 * b2, cells + b0 * b2, cells + b0 * b1};
-                double cta = 2.0 + VW * rounds(cells * C::QV) + 0.6 * rounds(cells * C::NPAIR);
-                for (int f : fd) cta += 2.0 * rounds(f * C::FQ) + 0.8 * rounds(2 * C::NG * f + C::NPAIR * cells);
-                const double waves = tile_waves(tiles, C::MINB);
-                const double cost = waves * cta;
-                if (cost < bc) {
-                    bc = cost;
-                    best.b[0] = b0;
-                    best.b[1] = b1;
-                    best.b[2] = b2;
-                    best.t[0] = (int)t0;
-                    best.t[1] = (int)t1;
-                    best.t[2] = (int)t2;
+    static thread_local TileMemo memo;
+    ModalTile t = memo.get({{0, 0, m0, n1, n2, 0}}, [&] {
+        ModalTile best{};
+        double bc = 1e300;
+        const int ext[] = {1, 2, 3, 4, 5, 6, 8};
+        for (int b0 : ext)
+            for (int b1 : ext)
+                for (int b2 : ext) {
+                    const int cells = b0 * b1 * b2;
+                    const int fmax = cells + std::max(b1 * b2, std::max(b0 * b2, b0 * b1));
+                    if (cells > C::CELLS || (b0 + 2) * (b1 + 2) * (b2 + 2) > C::SLOTS || fmax > C::FACES) continue;
+                    const long long t0 = (m0 + b0 - 1) / b0, t1 = (n1 + b1 - 1) / b1, t2 = (n2 + b2 - 1) / b2;
+                    const double tiles = (double)t0 * t1 * t2;
+                    // a CTA's time from the rounds of its phases (weights: measured shares, k = 2 and 4)
+                    auto rounds = [](int tasks) { return (double)((tasks + C::NT - 1) / C::NT); };
+                    const int fd[3] = {cells + b1 * b2, cells + b0 * b2, cells + b0 * b1};
+                    double cta = 2.0 + VW * rounds(cells * C::QV) + 0.6 * rounds(cells * C::NPAIR);
+                    for (int f : fd) cta += 2.0 * rounds(f * C::FQ) + 0.8 * rounds(2 * C::NG * f + C::NPAIR * cells);
+                    const double waves = tile_waves(tiles, C::MINB);
+                    const double cost = waves * cta;
+                    if (cost < bc) {
+                        bc = cost;
+                        best.b[0] = b0;
+                        best.b[1] = b1;
+                        best.b[2] = b2;
+                        best.t[0] = (int)t0;
+                        best.t[1] = (int)t1;
+                        best.t[2] = (int)t2;
+                    }
                 }
-            }
-    best.ncell = best.b[0] * best.b[1] * best.b[2];
-    memo.m0 = m0;
-    memo.n1 = n1;
-    memo.n2 = n2;
-    memo.t = best;
-    best.s0 = s0;
-    return best;
+        best.ncell = best.b[0] * best.b[1] * best.b[2];
+        return best;
+    });
+    t.s0 = s0;
+    return t;
 }
 
 template <int K, int Q, int MODE>

@@ -5,6 +5,8 @@
 // doubles in a (b+2)^3 halo box; the corners stay unused. The copies are asynchronous 8-byte
 // ones: the caller's vectors may start at any double.
 #pragma once
+#include <algorithm>
+
 #include "modal.h"
 
 namespace bosss {
@@ -27,6 +29,35 @@ inline double tile_waves(double tiles, int per_sm) {
     const double rest = sm <= 0.0 ? 0.0 : sm <= 1.0 ? (per_sm == 1 ? 1.0 : 0.6) : 0.6 + 0.4 * (sm - 1.0) / (per_sm - 1);
     return full + rest;
 }
+
+// Extents found for the last grids on one thread: they depend on the sizes alone, and the search over a
+// few hundred candidates costs as much as a launch. Several entries, replaced in turn, because callers
+// alternate between grids or ranges of one (species B of an XDG operator has up to three ranges); with one
+// entry, three small advection-diffusion grids in turn took 9.2 us per residual, with these 6.6
+class TileMemo {
+public:
+    struct Key {
+        int v[6];
+    };
+    template <class Search>
+    const ModalTile& get(const Key& k, Search&& search) {
+        for (int i = 0; i < used_; ++i)
+            if (std::equal(k.v, k.v + 6, key_[i].v)) return tile_[i];
+        const int i = next_;
+        next_ = (next_ + 1) % SIZE;
+        if (used_ < SIZE) ++used_;
+        tile_[i] = search();
+        key_[i] = k;
+        return tile_[i];
+    }
+
+    static constexpr int SIZE = 16;
+
+private:
+    Key key_[SIZE] = {};
+    ModalTile tile_[SIZE] = {};
+    int used_ = 0, next_ = 0;
+};
 
 // memory-order view of a three-dimensional grid and the block of one tile
 struct TileGeom {
