@@ -24,7 +24,7 @@
 #include "batch.h"
 #include "dg_slab_kernel.cuh"
 #include "handle.h"
-#include "modal.h"
+#include "modal_batch.h"
 
 namespace bosss {
 
@@ -678,10 +678,12 @@ int bosss_b200_batch_autotune(bosss_batch* b, const double* U_dev, const double*
             b->tiles[kq] = table[key];
             continue;
         }
+        // the modal path has one tile per CTA and no queue: nothing to time, and nothing to record
+        // for the queue batches that share the key
+        if (b->modal) continue;
         int best = 1;
         float best_ms = 1e30f;
         for (int r : {1, 2, 4, 8}) {
-            if (b->modal) break;   // one tile per CTA: nothing to time
             b->tiles[kq] = r;
             float ms = 0.f;
             rc = time_once(ms);
@@ -725,7 +727,7 @@ int bosss_b200_batch_autotune(bosss_batch* b, const double* U_dev, const double*
     if (table_path && *table_path) {
         std::ofstream f(table_path);
         for (auto& kv : table) f << kv.first << " " << kv.second << "\n";
-        f << "schedule " << (b->classes ? "classes" : (b->lpt ? "lpt" : "fifo")) << "\n";
+        if (have_sched || !b->modal) f << "schedule " << (b->classes ? "classes" : (b->lpt ? "lpt" : "fifo")) << "\n";
     }
     if (b->graph) {
         cudaGraphExecDestroy(b->graph);

@@ -1,11 +1,7 @@
 // modal.h -- modal stencil kernels of linear constant-coefficient scalar operators (modal.cu).
 #pragma once
-#include <vector>
-
 #include "dg_kernel.cuh"
 #include "dg_registry.h"
-
-struct bosss_handle;
 
 namespace bosss {
 
@@ -36,13 +32,5 @@ struct ModalItem {
 // tile extents for the cells [cbeg, cend) of a grid; `shared`: the launch holds other grids too,
 // so that this one need not spread over the whole chip
 ModalTile modal_tiling(const EvalArgs& a, int D, int K, bool shared = false);
-
-struct ModalBatch;
-// *out stays null (no error) where an instance does not qualify
-int modal_batch_create(const std::vector<bosss_handle*>& hs, const long long* dom_off, const long long* cod_off,
-                       ModalBatch** out);
-void modal_batch_destroy(ModalBatch* m);
-int modal_batch_run(const ModalBatch* m, int mode, double alpha, double beta, const double* U, const double* V,
-                    double* out, cudaStream_t s);
 
 }  // namespace bosss

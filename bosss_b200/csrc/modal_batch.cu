@@ -1,8 +1,9 @@
 // modal_batch.cu -- the modal stencil kernel over the instances of a batch: one launch per
 // degree, one tile of one instance per CTA. Batches whose instances are all linear with constant
 // coefficients (modal_applies) run here; others keep the quadrature tiles of batch.cu.
+#include "modal_batch.h"
+
 #include <algorithm>
-#include <vector>
 
 #include "handle.h"
 #include "modal_kernel.cuh"

@@ -1,0 +1,54 @@
+"""The work queue and the class launches of the batch (nonlinear instances and explicit kernel
+selectors; linear batches run on the modal kernel): the autotuner's table."""
+import numpy as np
+import pytest
+
+from bosss_b200 import _capi as C
+from bosss_b200 import operator as O
+from bosss_b200 import problems as P
+
+pytestmark = pytest.mark.gpu
+
+
+def linear_batch():
+    return P.batched_advection_diffusion(n_instances=6, seed=77, sizes=(3, 4, 5), degrees=(1, 2, 3))
+
+
+def nonlinear_batch():
+    """The same shape of batch; every second instance has nu(u) = nu0 + nu2 u^2."""
+    probs = linear_batch()
+    for i, p in enumerate(probs):
+        if i % 2 == 0:
+            op = O.DifferentialOperator(["u"], [], ["R"], O.QuadOrderFunc.Linear())
+            op.EquationComponents["R"].Add(O.ScalarTransportFlux(p.config["velocity"], "u"))
+            op.EquationComponents["R"].Add(O.SIPLaplace(4.0, "u", nu0=0.3, nu2=0.2))
+            op.Commit()
+            p.op = op
+    return probs
+
+
+def vectors(probs):
+    import torch
+    U = torch.from_numpy(np.concatenate([p.U for p in probs])).cuda()
+    W = torch.from_numpy(np.random.default_rng(4).uniform(-1, 1, U.numel())).cuda()
+    return U, W, torch.zeros_like(U), torch.zeros_like(U)
+
+
+@pytest.mark.parametrize("later", ["nonlinear", "generic", "slab"])
+def test_tuning_a_linear_batch_records_nothing_for_queue_batches(tmp_path, later):
+    """The modal path has nothing to time: the table keeps what it held, and a queue batch of the same
+    classes is tuned when it comes."""
+    table = tmp_path / "tiles.txt"
+    table.write_text("phys9_D3_K9_Q9 4\n")
+    probs = linear_batch()
+    with O.BatchEvaluator(probs) as b:
+        b.autotune(*vectors(probs), str(table))
+    assert table.read_text().split() == ["phys9_D3_K9_Q9", "4"]
+    probs = nonlinear_batch() if later == "nonlinear" else probs
+    kernel = {"nonlinear": C.KERNEL_AUTO, "generic": C.KERNEL_GENERIC, "slab": C.KERNEL_SLAB}[later]
+    with O.BatchEvaluator(probs, kernel=kernel) as b:
+        b.autotune(*vectors(probs), str(table))
+    text = table.read_text()
+    for k in {p.dom[0].degree for p in probs}:
+        assert "_D3_K%d_Q%d" % (k, k + 1) in text      # tuned and recorded
+    assert text.splitlines()[-1].split()[0] == "schedule"
