@@ -482,6 +482,20 @@ int bosss_b200_batch_create(int32_t n, const bosss_op_desc* ops, const bosss_gri
     };
     cudaError_t e = cudaSetDevice(b->device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
+    if (e != cudaSuccess) return bail(e);
+    // linear instances with constant coefficients: the modal kernel; the work queue and the class
+    // lists are built for the others only
+    if (want == 0) {
+        const int rc = modal_batch_create(b->h, b->dom_off.data(), b->cod_off.data(), &b->modal);
+        if (rc) {
+            bosss_b200_batch_destroy(b);
+            return rc;
+        }
+    }
+    if (b->modal) {
+        *out = b;
+        return BOSSS_OK;
+    }
     std::vector<BatchInst> hi(n);
     for (int i = 0; i < n; ++i) {
         hi[i].a = b->h[i]->base;
@@ -490,7 +504,7 @@ int bosss_b200_batch_create(int32_t n, const bosss_op_desc* ops, const bosss_gri
         hi[i].K = b->h[i]->K;
         hi[i].Q = b->h[i]->Q;
     }
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_inst, sizeof(BatchInst) * n);
+    e = cudaMalloc(&b->d_inst, sizeof(BatchInst) * n);
     if (e == cudaSuccess) e = cudaMemcpy(b->d_inst, hi.data(), sizeof(BatchInst) * n, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_counter, sizeof(int) * 2);
     if (e != cudaSuccess) return bail(e);
@@ -498,13 +512,6 @@ int bosss_b200_batch_create(int32_t n, const bosss_op_desc* ops, const bosss_gri
         b->grid[m] = batch_grid(b->phys, m, b->slab[m]);
         int rc = build_items(b, m);
         if (!rc) rc = build_class_items(b, m, want);
-        if (rc) {
-            bosss_b200_batch_destroy(b);
-            return rc;
-        }
-    }
-    if (want == 0) {
-        const int rc = modal_batch_create(b->h, b->dom_off.data(), b->cod_off.data(), &b->modal);
         if (rc) {
             bosss_b200_batch_destroy(b);
             return rc;
@@ -719,7 +726,7 @@ int bosss_b200_batch_autotune(bosss_batch* b, const double* U_dev, const double*
             b->lpt = rc ? true : (ms_l <= ms_f);
             b->classes = !rc && ms_c < std::min(ms_l, ms_f);
         }
-        for (int m = 0; m < 3 && !rc; ++m) rc = build_items(b, m);
+        for (int m = 0; m < 3 && !rc && !b->modal; ++m) rc = build_items(b, m);
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);

@@ -52,3 +52,18 @@ def test_tuning_a_linear_batch_records_nothing_for_queue_batches(tmp_path, later
     for k in {p.dom[0].degree for p in probs}:
         assert "_D3_K%d_Q%d" % (k, k + 1) in text      # tuned and recorded
     assert text.splitlines()[-1].split()[0] == "schedule"
+
+
+def test_linear_batches_build_no_queue():
+    """Work items and class lists (24 bytes per tile, mode and list) are not built for a batch that
+    never reads them."""
+    import torch
+    probs = [P.advection_diffusion3d(n=32, k=4, seed=5, velocity=(0.3, -0.2, 0.5))] * 32    # 1.05e6 cells
+
+    def device_bytes():
+        free0 = torch.cuda.mem_get_info()[0]
+        with O.BatchEvaluator(probs):
+            return free0 - torch.cuda.mem_get_info()[0]
+
+    device_bytes()                    # kernels loaded
+    assert device_bytes() <= 6 << 20  # the lists take 10 MB here
