@@ -11,12 +11,8 @@ namespace {
 
 template <class C>
 ModalTile euler_tiling(const EvalArgs& a) {
-    const GridConst& g = a.g;
-    const bool rev = g.stride[0] == 1 && g.stride[2] != 1;
-    const int n0 = rev ? g.n[2] : g.n[0], n1 = g.n[1], n2 = rev ? g.n[0] : g.n[2];
-    const long long plane = (long long)n1 * n2;
-    const int s0 = (int)(a.cbeg / plane), s1 = (int)std::min<long long>(n0, (a.cend + plane - 1) / plane);
-    const int m0 = std::max(1, s1 - s0);
+    const TileRange r = tile_range(a, 3);
+    const int m0 = r.planes, n1 = r.n[1], n2 = r.n[2];
     static thread_local TileMemo memo;
     ModalTile t = memo.get({{0, 0, m0, n1, n2, 0}}, [&] {
         ModalTile best{};
@@ -51,7 +47,8 @@ ModalTile euler_tiling(const EvalArgs& a) {
         best.ncell = best.b[0] * best.b[1] * best.b[2];
         return best;
     });
-    t.s0 = s0;
+    t.s0 = r.s0;
+    t.planes = r.planes;
     return t;
 }
 

@@ -3,7 +3,6 @@
 #include <algorithm>
 
 #include "modal_kernel.cuh"
-#include "tile_stage.cuh"
 
 namespace bosss {
 
@@ -70,12 +69,8 @@ KernelEntry modal_entry(int phys, int D, int K, int mode) {
 }
 
 ModalTile modal_tiling(const EvalArgs& a, int D, int K, bool shared) {
-    const GridConst& g = a.g;
-    const bool rev = D == 3 && g.stride[0] == 1 && g.stride[2] != 1;
-    const int n0 = rev ? g.n[2] : g.n[0], n1 = D == 3 ? g.n[1] : 1, n2 = D == 3 ? (rev ? g.n[0] : g.n[2]) : g.n[1];
-    const long long plane = (long long)n1 * n2;
-    const int s0 = (int)(a.cbeg / plane), s1 = (int)std::min<long long>(n0, (a.cend + plane - 1) / plane);
-    const int m0 = std::max(1, s1 - s0);
+    const TileRange r = tile_range(a, D);
+    const int m0 = r.planes, n1 = r.n[1], n2 = r.n[2];
     int cells = 0, box = 0, per_sm = 1;
     auto cfg = [&](auto c) {
         using C = decltype(c);
@@ -125,7 +120,8 @@ ModalTile modal_tiling(const EvalArgs& a, int D, int K, bool shared) {
         best.ncell = best.b[0] * best.b[1] * best.b[2];
         return best;
     });
-    t.s0 = s0;
+    t.s0 = r.s0;
+    t.planes = r.planes;
     return t;
 }
 

@@ -23,7 +23,7 @@ KernelEntry modal_entry(int phys, int D, int K, int mode);
 struct ModalTile {
     int b[3];        // tile extent in memory order (slow, middle, fast); 2D: middle = 1
     int t[3];        // tiles per memory direction
-    int s0;          // first plane of the slowest direction
+    int s0, planes;  // first plane of the slowest direction and number of planes that hold the launch's cells
     int ncell;       // b[0] * b[1] * b[2]
 };
 struct ModalItem {

@@ -30,7 +30,7 @@
 // Poisson 80^3 k = 2 (both species, cut items and interface) 1.72 -> 0.29 ms, cut items and
 // interface (also rewritten) 0.12 ms of it.
 #pragma once
-#include "modal.h"
+#include "tile_stage.cuh"
 
 namespace bosss {
 
@@ -330,15 +330,12 @@ __device__ __forceinline__ void modal_tile(const EvalArgs& a, const Tables1D& T,
     const GridConst& g = a.g;
     const int tid = threadIdx.x;
     // memory directions: generator order x slow .. z fast; GlobalID order the other way round
-    const bool rev = (D == 3) && g.stride[0] == 1 && g.stride[2] != 1;
-    const int n0 = rev ? g.n[2] : g.n[0], n1 = (D == 3) ? g.n[1] : 1, n2 = (D == 3) ? (rev ? g.n[0] : g.n[2]) : g.n[1];
-    const int per0 = rev ? g.periodic[2] : g.periodic[0], per1 = (D == 3) ? g.periodic[1] : 0;
-    const int per2 = (D == 3) ? (rev ? g.periodic[0] : g.periodic[2]) : g.periodic[1];
-    const int b0 = tl.b[0], b1 = tl.b[1], b2 = tl.b[2];
-    const int t2 = tile % tl.t[2], tq = tile / tl.t[2];
-    const int t1 = tq % tl.t[1], t0 = tq / tl.t[1];
-    const int o0 = tl.s0 + t0 * b0, o1 = t1 * b1, o2 = t2 * b2;
-    const int e0 = min(b0, n0 - o0), e1 = min(b1, n1 - o1), e2 = min(b2, n2 - o2);
+    const TileGeom G = tile_geom<D>(g, tl, tile);
+    const bool rev = G.rev;
+    const int n0 = G.n[0], n1 = G.n[1], n2 = G.n[2];
+    const int per0 = G.per[0], per1 = G.per[1], per2 = G.per[2];
+    const int b1 = tl.b[1], b2 = tl.b[2];
+    const int o0 = G.o[0], o1 = G.o[1], o2 = G.o[2], e0 = G.e[0], e1 = G.e[1], e2 = G.e[2];
     // slots: halo box, fast direction innermost
     const int w2 = b2 + 2, w1 = (D == 3) ? b1 + 2 : 1;
     const int q1 = w2, q0 = w1 * w2;

@@ -59,7 +59,25 @@ private:
     int used_ = 0, next_ = 0;
 };
 
-// memory-order view of a three-dimensional grid and the block of one tile
+// memory-order extents of a grid (slow, middle, fast; 2D: middle = 1), first plane of the slow direction
+// and number of planes that hold the cells [cbeg, cend)
+struct TileRange {
+    int n[3], s0, planes;
+};
+inline TileRange tile_range(const EvalArgs& a, int D) {
+    const GridConst& g = a.g;
+    const bool rev = D == 3 && g.stride[0] == 1 && g.stride[2] != 1;
+    TileRange r;
+    r.n[0] = rev ? g.n[2] : g.n[0];
+    r.n[1] = D == 3 ? g.n[1] : 1;
+    r.n[2] = D == 3 ? (rev ? g.n[0] : g.n[2]) : g.n[1];
+    const long long plane = (long long)r.n[1] * r.n[2];
+    r.s0 = (int)(a.cbeg / plane);
+    r.planes = (int)std::max<long long>(1, std::min<long long>(r.n[0], (a.cend + plane - 1) / plane) - r.s0);
+    return r;
+}
+
+// memory-order view of a grid and the block of one tile
 struct TileGeom {
     bool rev;          // GlobalID order: x fastest
     int n[3], per[3];  // cells and periodicity per memory direction
@@ -70,21 +88,26 @@ struct TileGeom {
     __device__ __forceinline__ int mem(int d) const { return rev ? 2 - d : d; }
 };
 
-__device__ __forceinline__ TileGeom tile_geom(const GridConst& g, const ModalTile& tl, int tile) {
+// The block ends with the launch's planes, not with the grid: beyond the range only the face neighbours of
+// its cells are read, so that a caller may still be writing the rest (host chunks that are on their way,
+// a halo exchange in flight)
+template <int D = 3>
+__host__ __device__ __forceinline__ TileGeom tile_geom(const GridConst& g, const ModalTile& tl, int tile) {
     TileGeom G;
-    G.rev = g.stride[0] == 1 && g.stride[2] != 1;
+    G.rev = D == 3 && g.stride[0] == 1 && g.stride[2] != 1;
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
-        G.n[m] = G.rev ? g.n[2 - m] : g.n[m];
-        G.per[m] = G.rev ? g.periodic[2 - m] : g.periodic[m];
+        G.n[m] = D == 2 ? (m == 1 ? 1 : g.n[m >> 1]) : G.rev ? g.n[2 - m] : g.n[m];
+        G.per[m] = D == 2 ? (m == 1 ? 0 : g.periodic[m >> 1]) : G.rev ? g.periodic[2 - m] : g.periodic[m];
     }
     const int t2 = tile % tl.t[2], tq = tile / tl.t[2];
     const int t1 = tq % tl.t[1], t0 = tq / tl.t[1];
     G.o[0] = tl.s0 + t0 * tl.b[0];
     G.o[1] = t1 * tl.b[1];
     G.o[2] = t2 * tl.b[2];
-#pragma unroll
-    for (int m = 0; m < 3; ++m) G.e[m] = min(tl.b[m], G.n[m] - G.o[m]);
+    G.e[0] = min(tl.b[0], tl.planes - t0 * tl.b[0]);   // (from a plane's number: more registers, SIP 2 % slower)
+    G.e[1] = min(tl.b[1], G.n[1] - G.o[1]);
+    G.e[2] = min(tl.b[2], G.n[2] - G.o[2]);
     G.q1 = tl.b[2] + 2;
     G.q0 = (tl.b[1] + 2) * (tl.b[2] + 2);
     return G;

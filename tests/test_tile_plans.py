@@ -1,5 +1,5 @@
 """Tile plans of the block kernels on the host: ``tests/native/tile_plan_check.cu`` is compiled by nvcc
-as host code and checks the memo of the extents."""
+as host code and checks the memo of the extents and the cells that the blocks of a cell range cover."""
 import os
 import shutil
 import subprocess
