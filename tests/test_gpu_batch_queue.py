@@ -1,13 +1,19 @@
 """The work queue and the class launches of the batch (nonlinear instances and explicit kernel
-selectors; linear batches run on the modal kernel): the autotuner's table."""
+selectors; linear batches run on the modal kernel): every schedule against the oracle and the single
+instances, the captured step, and the autotuner's table."""
 import numpy as np
 import pytest
 
 from bosss_b200 import _capi as C
 from bosss_b200 import operator as O
 from bosss_b200 import problems as P
+from oracle import oracle as orc
 
 pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-300)
 
 
 def linear_batch():
@@ -67,3 +73,59 @@ def test_linear_batches_build_no_queue():
 
     device_bytes()                    # kernels loaded
     assert device_bytes() <= 6 << 20  # the lists take 10 MB here
+
+
+KINDS = {"generic": (linear_batch, C.KERNEL_GENERIC), "slab": (linear_batch, C.KERNEL_SLAB),
+         "nonlinear": (nonlinear_batch, C.KERNEL_AUTO)}
+
+
+@pytest.mark.parametrize("schedule", ["classes", "lpt", "fifo"])
+@pytest.mark.parametrize("kind", sorted(KINDS))
+def test_queue_schedules_match_oracle_and_single_instances(tmp_path, kind, schedule):
+    import torch
+    make, kernel = KINDS[kind]
+    probs = make()
+    U, W, R, G = vectors(probs)
+    table = tmp_path / "tiles.txt"
+    table.write_text("schedule %s\n" % schedule)
+    with O.BatchEvaluator(probs, kernel=kernel) as b:
+        b.autotune(U, W, R, G, str(table))
+        assert b.tiles(1, 2)[1] == schedule
+        out = [b.evaluate(m, U, None if m == C.MODE_RESIDUAL else W) for m in range(3)]
+        torch.cuda.synchronize()
+        off = b.dom_offsets
+    for i, p in enumerate(probs):
+        sl = slice(int(off[i]), int(off[i + 1]))
+        got = [t[sl].cpu().numpy() for t in out]
+        w = W[sl].cpu().numpy()
+        ref = [orc.evaluate(*p.descs(), p.U), orc.jvp(*p.descs(), p.U, w), orc.vjp(*p.descs(), p.U, w)]
+        for a, r in zip(got, ref):
+            assert rel(a, r) <= 1e-12
+        if kind != "nonlinear":       # the tiles of the single-grid kernel
+            with p.evaluator(kernel=kernel) as ev:
+                single = np.zeros(p.n_dofs)
+                ev.Evaluate(1.0, 0.0, single, p.U)
+                for a, r in zip(got, (single, ev.jvp(p.U, w), ev.vjp(p.U, w))):
+                    assert rel(a, r) <= 1e-13
+
+
+@pytest.mark.parametrize("kind", sorted(KINDS))
+def test_queue_graph_replay_and_autotune(tmp_path, kind):
+    import torch
+    make, kernel = KINDS[kind]
+    probs = make()
+    U, W, R, G = vectors(probs)
+    table = str(tmp_path / "tiles.txt")
+    with O.BatchEvaluator(probs, kernel=kernel) as b:
+        Rd, Gd = b.evaluate(C.MODE_RESIDUAL, U), b.evaluate(C.MODE_VJP, U, W)
+        b.autotune(U, W, R, G, table)
+        b.capture(U, W, R, G)
+        R.zero_()
+        G.zero_()
+        b.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(R, Rd) and torch.equal(G, Gd)
+        tiles = {k: b.tiles(k, k + 1) for k in (1, 2, 3)}
+    with O.BatchEvaluator(probs, kernel=kernel) as b2:      # reads the table instead of timing again
+        b2.autotune(U, W, R, G, table)
+        assert {k: b2.tiles(k, k + 1) for k in tiles} == tiles

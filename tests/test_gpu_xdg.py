@@ -251,3 +251,27 @@ def test_caller_length_scales_take_effect(xdg_small):
     finally:
         X.set_length_scales(s, None)
     assert np.array_equal(np.nan_to_num(X.length_scales(s), nan=-1), np.nan_to_num(base, nan=-1))
+
+
+@pytest.mark.parametrize("kind", ["modal", "slab", "slab_of_nonlinear"])
+def test_xdg_masked_bulk_kernels_equal_masked_generic(kind):
+    """Every bulk kernel that reads the species masks (modal and slab of the constant-viscosity bulk, the
+    slab that nonlinear handles fall back to, Q = 2K + 1) against the masked generic tile."""
+    opA, opB, g, c, UA, UB = small_case(n=12)
+    if kind == "slab_of_nonlinear":
+        ops = []
+        for mu in (1.0, 10.0):
+            op = O.DifferentialOperator(["u"], [], ["R"], O.QuadOrderFunc.NonLinear(3))
+            op.EquationComponents["R"].Add(O.SIPLaplace(4.0, "u", nu0=mu, nu2=0.3))
+            op.EquationComponents["R"].Add(O.ConstantSource(1.0, "u"))
+            op.Commit()
+            ops.append(op)
+        opA, opB = ops
+    kernel = C.KERNEL_SLAB if kind == "slab" else C.KERNEL_AUTO
+    with O.XdgEvaluator(opA, opB, g, 2, c, 0.4, kernel=kernel) as Xs, O.XdgEvaluator(opA, opB, g, 2, c, 0.4,
+                                                                                    kernel=C.KERNEL_GENERIC) as Xg:
+        for s, U in enumerate((UA, UB)):
+            a, b = np.zeros_like(U), np.zeros_like(U)
+            Xs.Evaluate(s, 1.0, 0.0, a, U)
+            Xg.Evaluate(s, 1.0, 0.0, b, U)
+            assert rel(a, b) <= 1e-13, (s, rel(a, b))
