@@ -913,7 +913,8 @@ static int host_pipelined(bosss_handle* h, const HostJob* jobs, int njobs, const
         }
     }
     // later calls on the handle's stream follow the second stream's work as well
-    if (two) CUDA_TRY(cudaStreamWaitEvent(s, h->ev_second[nch - 1], 0));
+    if (two) e = cudaStreamWaitEvent(s, h->ev_second[nch - 1], 0);
+    if (e != cudaSuccess) return finish(fail(BOSSS_ERR_CUDA, cudaGetErrorString(e)));
     if (h->check_nan)
         for (int k = 0; k < njobs; ++k) {
             rc = check_nan(h, jobs[k].dY, nY(jobs[k]) * J, s);
