@@ -54,7 +54,7 @@ struct EulerCfg {
     static constexpr int O_TAB = 0, O_COEF = 2 * Q * (K + 1) + Q + 1;
     static constexpr int O_R = O_COEF + NG * CELLS * S, O_WORK = O_R + NC * CST;
     static constexpr size_t SMEM = sizeof(double) * (O_WORK + WORK);
-    };
+};
 
 __device__ constexpr double kEulE[5] = {0.70710678118654752440, 1.22474487139158904910, 1.58113883008418966600,
                                         1.87082869338697069279, 2.12132034355964257320};

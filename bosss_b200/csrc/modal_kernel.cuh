@@ -34,7 +34,6 @@
 
 namespace bosss {
 
-
 template <int D, int K>
 struct ModalCfg {
     static constexpr int NP = np_of(D, K);
@@ -97,28 +96,6 @@ struct FaceCoef {
     double cO, cN, p, hO, hN, k;
 };
 
-__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
-}
-
-// 1 / cell length scale of a cell (penalty_size without divisions)
-__device__ __forceinline__ double modal_size(const EvalArgs& a, const int* ijk) {
-    if (a.cell_pf) return penalty_size(a.cell_pf, a.g, ijk);
-    double cj = 0.0;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        if (d >= a.g.D) break;
-        int nb = 2;
-        if (!a.g.gper[d]) {
-            const int gi = ijk[d] + a.g.goff[d];
-            nb += (gi == 0) + (gi == a.g.gn[d] - 1);
-        }
-        cj += nb * (0.5 * a.g.twoh[d]);
-    }
-    return 0.5 * cj;
-}
-
 // coefficients of face (dir, s) of cell ijk; nb: there is a neighbour whose coefficients enter
 template <int D, bool SIP, int MODE>
 __device__ __forceinline__ FaceCoef modal_face(const EvalArgs& a, const int* ijk, int dir, int s, bool on, bool& nb) {
@@ -141,7 +118,7 @@ __device__ __forceinline__ FaceCoef modal_face(const EvalArgs& a, const int* ijk
         if constexpr (SIP) {
             int ijk2[3] = {ijk[0], ijk[1], ijk[2]};
             ijk2[dir] = i;
-            p = sip ? a.ph.pen * fmax(modal_size(a, ijk), modal_size(a, ijk2)) * nu : 0.0;
+            p = sip ? a.ph.pen * fmax(tile_size<D>(a, ijk), tile_size<D>(a, ijk2)) * nu : 0.0;
         }
         if (MODE == MODE_VJP) {
             f.p = p - (s ? ap : -am);   // both sides of the upwind flux see the jump of w
@@ -156,7 +133,7 @@ __device__ __forceinline__ FaceCoef modal_face(const EvalArgs& a, const int* ijk
         const double an = s ? vel : -vel;
         if (tr && (D == 2 || an >= 0.0)) f.cO = an;
         if (sip && a.ph.dirichlet) {
-            f.p = 2.0 * a.ph.pen * modal_size(a, ijk) * nu;
+            f.p = 2.0 * a.ph.pen * tile_size<D>(a, ijk) * nu;
             f.hO = nu * th;
             f.k = nu;
         }
@@ -410,7 +387,7 @@ __device__ __forceinline__ void modal_tile(const EvalArgs& a, const Tables1D& T,
             const int o = e + (S - NP) * (e / NP);
 #pragma unroll
             for (int k = 0; k < C::GRP; ++k)
-                if (e < n[k]) cp_async8(sm + dst[k] + o, src[k] + e);
+                if (e < n[k]) tile_cp8(sm + dst[k] + o, src[k] + e);
         }
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");

@@ -446,7 +446,8 @@ __global__ void k_dense_apply(int N, const double* __restrict__ M, const double*
 
 int launch_grid(long long n) { return (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, 148LL * 16)); }
 
-// the number of scalar rows of a p-level fits 32 bits (J <= 2e9 cells would need 8 m TB of blocks)
+// the number J m of scalar rows of a p-level fits 32 bits: at 2^32 the level's blocks alone, at least
+// 5 m^2 doubles for each of the J cells, would take 515 GB (m = 3; more for larger m)
 void launch_bdiag(long long J, int m, const double* inv, const double* in, double* out, int add, cudaStream_t s) {
     const unsigned n = (unsigned)(J * m);
     const int gr = launch_grid(J * m);
@@ -514,7 +515,10 @@ struct bosss_pmg {
     static size_t padded(size_t n) { return (std::max<size_t>(n, 1) + 31) / 32 * 32; }
     bool reserve(size_t n) {
         void* p = nullptr;
-        if (cudaMalloc(&p, sizeof(double) * n) != cudaSuccess) return false;
+        if (cudaMalloc(&p, sizeof(double) * n) != cudaSuccess) {
+            cudaGetLastError();   // or the next launch would report it
+            return false;
+        }
         owned.push_back(p);
         block = (double*)p;
         left = n;
@@ -522,10 +526,7 @@ struct bosss_pmg {
     }
     double* alloc(size_t n) {
         n = padded(n);
-        if (n > left) {
-            cudaGetLastError();
-            return nullptr;
-        }
+        if (n > left) return nullptr;
         double* p = block;
         block += n;
         left -= n;

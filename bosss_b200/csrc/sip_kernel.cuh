@@ -54,24 +54,8 @@ __device__ __forceinline__ constexpr int sip_mode(int m, int p, int r) {
     return DIR == 0 ? mode3(m, p, r) : (DIR == 1 ? mode3(p, m, r) : mode3(p, r, m));
 }
 
-// 1 / cell length scale of a cell (penalty_size without divisions)
-__device__ __forceinline__ double sip_size(const EvalArgs& a, const int* ijk) {
-    if (a.cell_pf) return penalty_size(a.cell_pf, a.g, ijk);
-    double cj = 0.0;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        int nb = 2;
-        if (!a.g.gper[d]) {
-            const int gi = ijk[d] + a.g.goff[d];
-            nb += (gi == 0) + (gi == a.g.gn[d] - 1);
-        }
-        cj += nb * (0.5 * a.g.twoh[d]);
-    }
-    return 0.5 * cj;
-}
-
 // one row of a contraction over y and z: rv[a] = sum_bc c[abc] Ay[b] Az[c], and its y / z derivatives
-template <int K, bool VAL>
+template <int K>
 __device__ __forceinline__ void sip_rows(const double* c, const double* Ay, const double* dAy, const double* Az,
                                          const double* dAz, double* rv, double* ry, double* rz) {
 #pragma unroll
@@ -208,7 +192,7 @@ __device__ __forceinline__ void sip_face_rows(const EvalArgs& a, const TileGeom&
                                               int fd1, int fd2) {
     using C = SipCfg<K, Q, MODE>;
     constexpr int t1 = (DIR == 0) ? 1 : 0, t2 = (DIR == 2) ? 1 : 2;
-    const int nf = fd0 * fd1 * fd2, md = G.mem(DIR);
+    const int nf = fd0 * fd1 * fd2;
     const Tables1D& T = a.tab;
     const double vel = a.ph.has_transport ? a.ph.vel[DIR] : 0.0;
     const bool sip = a.ph.has_sip != 0;
@@ -225,7 +209,6 @@ __device__ __forceinline__ void sip_face_rows(const EvalArgs& a, const TileGeom&
             ijk[1] = m1;
             ijk[2] = G.rev ? m0 : m2;
         }
-        (void)md;
         const int gi = ijk[DIR];
         const bool per = a.g.periodic[DIR] != 0;
         const bool hasA = gi > 0 || per, hasB = gi < nn || per;
@@ -259,7 +242,7 @@ __device__ __forceinline__ void sip_face_rows(const EvalArgs& a, const TileGeom&
                 int iA[3] = {ijk[0], ijk[1], ijk[2]}, iB[3] = {ijk[0], ijk[1], ijk[2]};
                 iA[DIR] = gi > 0 ? gi - 1 : nn - 1;
                 iB[DIR] = gi < nn ? gi : 0;
-                pnl = a.ph.pen * fmax(sip_size(a, iA), sip_size(a, iB));
+                pnl = a.ph.pen * fmax(tile_size<3>(a, iA), tile_size<3>(a, iB));
             }
 #pragma unroll
             for (int q1 = 0; q1 < Q; ++q1) {
@@ -289,7 +272,7 @@ __device__ __forceinline__ void sip_face_rows(const EvalArgs& a, const TileGeom&
             const bool dir = sip && a.ph.dirichlet;
             int io[3] = {ijk[0], ijk[1], ijk[2]};
             io[DIR] = hasA ? gi - 1 : gi;
-            const double pnl = sip ? 2.0 * a.ph.pen * sip_size(a, io) : 0.0;
+            const double pnl = sip ? 2.0 * a.ph.pen * tile_size<3>(a, io) : 0.0;
             const double xn = a.g.lo[DIR] + (gi + a.g.goff[DIR]) * a.g.h[DIR];
             const double x2 = a.g.lo[t2] + (io[t2] + a.g.goff[t2] + 0.5 + 0.5 * T.xq[q2]) * a.g.h[t2];
             const double gc = a.ph.g0 + (a.ph.g1[DIR] + a.ph.g2[DIR] * xn) * xn + (a.ph.g1[t2] + a.ph.g2[t2] * x2) * x2;
@@ -410,8 +393,8 @@ __device__ __forceinline__ void sip_volume(const EvalArgs& a, const Tables1D& V,
                 dAy[b] = V.dA[qy][b] * ty;
             }
             double uv[K + 1], uy[K + 1], uz[K + 1], wv[K + 1], wy[K + 1], wz[K + 1];
-            sip_rows<K, true>(cu, Ay, dAy, Az, dAz, uv, uy, uz);
-            if constexpr (C::NG > 1) sip_rows<K, true>(cv, Ay, dAy, Az, dAz, wv, wy, wz);
+            sip_rows<K>(cu, Ay, dAy, Az, dAz, uv, uy, uz);
+            if constexpr (C::NG > 1) sip_rows<K>(cv, Ay, dAy, Az, dAz, wv, wy, wz);
             double P[K + 1], Py[K + 1], Pz[K + 1];
 #pragma unroll
             for (int b = 0; b <= K; ++b) P[b] = Py[b] = Pz[b] = 0.0;
@@ -466,12 +449,11 @@ __device__ __forceinline__ void sip_volume(const EvalArgs& a, const Tables1D& V,
                 }
             }
             int pr = 0;
-            const double ity = 1.0;
 #pragma unroll
             for (int p = 0; p <= K; ++p)
 #pragma unroll
                 for (int b = 0; b <= K - p; ++b, ++pr) {
-                    P2[pr] += P[p] * Ay[b] + Py[p] * (V.dA[qy][b] * ity);
+                    P2[pr] += P[p] * Ay[b] + Py[p] * V.dA[qy][b];
                     P2z[pr] += Pz[p] * Ay[b];
                 }
         }

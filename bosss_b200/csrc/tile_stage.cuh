@@ -19,6 +19,23 @@ __device__ __forceinline__ void tile_cp_wait() {
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
 }
 
+// 1 / cell length scale of a cell (penalty_size without divisions)
+template <int D>
+__device__ __forceinline__ double tile_size(const EvalArgs& a, const int* ijk) {
+    if (a.cell_pf) return penalty_size(a.cell_pf, a.g, ijk);
+    double cj = 0.0;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+        int nb = 2;
+        if (!a.g.gper[d]) {
+            const int gi = ijk[d] + a.g.goff[d];
+            nb += (gi == 0) + (gi == a.g.gn[d] - 1);
+        }
+        cj += nb * (0.5 * a.g.twoh[d]);
+    }
+    return 0.5 * cj;
+}
+
 // Time of `tiles` CTAs in units of one CTA's time in a full wave of 148 x per_sm: whole waves, and for
 // the rest the pace of an SM that holds fewer CTAs (a CTA alone on its SM runs at about 0.6 of its
 // time among three); many waves overlap and count by their share
