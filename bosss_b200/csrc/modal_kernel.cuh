@@ -26,7 +26,7 @@
 // of 32 cells covers all banks; results leave in runs of consecutive cells.
 //
 // Measured on B200 against the quadrature tiles: advection-diffusion 20x31x27 k = 3, residual + JVP +
-// VJP 496 -> 31 us; 16 instances of 16^3..32^3, k = 1..4, residual + VJP 3.71 -> 0.148 ms; XDG
+// VJP 496 -> 31 us; 16 instances of 16^3..32^3, k = 1..4, residual + VJP 3.71 -> 0.146 ms; XDG
 // Poisson 80^3 k = 2 (both species, cut items and interface) 1.72 -> 0.29 ms, cut items and
 // interface (also rewritten) 0.12 ms of it.
 #pragma once

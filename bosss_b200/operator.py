@@ -655,7 +655,10 @@ class Evaluator:
 
 
 class BatchEvaluator:
-    """Independent operator instances evaluated by one persistent launch per mode.
+    """Independent operator instances evaluated together. Batches whose instances are all linear
+    with constant coefficients: one launch of the modal kernel per degree and mode. Others (or
+    with an explicit ``kernel``): one persistent launch per mode, or one launch per (degree,
+    rule) class, as :meth:`autotune` finds faster.
 
     ``problems``: list of objects with ``descs()`` (operator and grid descriptors), e.g.
     :class:`bosss_b200.problems.Problem`. Vectors are the concatenation of the
@@ -732,13 +735,16 @@ class BatchEvaluator:
         C.check(C.lib().bosss_b200_batch_replay(self.handle, ctypes.c_void_p(s if s else C.CUDA_STREAM_LEGACY)))
 
     def autotune(self, U, W, R, G, table_path=None):
+        """Time the queue's schedules on these vectors and record them in the table, or take them
+        from it. A linear batch has nothing to time and records nothing."""
         C.check(C.lib().bosss_b200_batch_autotune(self.handle, C.ptr(U), C.ptr(W), C.ptr(R), C.ptr(G),
                                                   table_path.encode() if table_path else None))
 
     SCHEDULES = {0: "fifo", 1: "lpt", 2: "classes"}
 
     def tiles(self, K, Q):
-        """(tiles per work item of the (K, Q) class, schedule: "lpt" | "fifo" | "classes")."""
+        """(tiles per work item of the (K, Q) class, schedule: "lpt" | "fifo" | "classes"); a linear
+        batch has no queue and returns what the table said, or the defaults."""
         t, sched = ctypes.c_int32(), ctypes.c_int32()
         C.check(C.lib().bosss_b200_batch_tiles(self.handle, K, Q, ctypes.byref(t), ctypes.byref(sched)))
         return t.value, BatchEvaluator.SCHEDULES[sched.value]

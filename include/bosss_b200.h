@@ -345,13 +345,16 @@ int bosss_b200_compute_jacobian(bosss_handle* h, const double* U, double time, b
 /* ---- batched evaluation ----
  * Many independent operator instances (own grid, DG degree and quadrature rule each,
  * same physics family; device path: 3D scalar transport / advection-diffusion) evaluated
- * by ONE persistent launch per mode: CTAs pull (instance, cell tile) work items from a
+ * together. With the automatic kernel (opt->kernel = 0) and instances that are all linear with
+ * constant coefficients: one launch of the modal kernel per degree and mode. Otherwise by ONE
+ * persistent launch per mode: CTAs pull (instance, cell tile) work items from a
  * queue in device memory. Vectors are the concatenation of the instances' vectors
  * (offsets from bosss_b200_batch_get_sizes). The residual + VJP pair can be captured once
- * into a CUDA graph and replayed; an autotuner picks the cell tiles per work item for each
- * (degree, quadrature nodes) class and the queue order, persisted in a small text table.
- * Tile kernel per mode (opt->kernel): 0 = automatic (register-blocked slab tiles when every
- * instance has at most 5 nodes per direction; else the generic tiles),
+ * into a CUDA graph and replayed; for the queue an autotuner picks the cell tiles per work item for
+ * each (degree, quadrature nodes) class and the queue order, persisted in a small text table (a
+ * batch on the modal kernel has nothing to time and records nothing).
+ * Tile kernel of the queue per mode (opt->kernel): 0 = automatic (register-blocked slab tiles when
+ * every instance has at most 5 nodes per direction; else the generic tiles),
  * 1 = generic tiles, 2 = slab tiles wherever every instance allows them. */
 typedef struct bosss_batch bosss_batch;
 
