@@ -303,6 +303,9 @@ __device__ __forceinline__ void eul_vol_project(const Tables1D& t, const double*
     }
 }
 
+// The node rounds r of a warp are separate code, and with two cells per warp (k = 2) a cell's nodes fall into other
+// rounds by its place in the block: every contraction is written out as fma, or the compiler's choice (which of two
+// products it fuses) would differ between rounds and a cell's bits would depend on the block it lies in
 template <int K, int MODE>
 __device__ __forceinline__ void eul_volume(const EvalArgs& a, const double* tA, const double* tdA, const double* tw,
                                            const double* coef, double* work, double* R, int ncell) {
@@ -354,13 +357,13 @@ __device__ __forceinline__ void eul_volume(const EvalArgs& a, const double* tA, 
             for (int r = 0; r < NR; ++r) {
                 const double ir = 1.0 / u[r][0];
                 const double v0 = u[r][1] * ir, v1 = u[r][2] * ir, v2 = u[r][3] * ir;
-                const double kin = u[r][1] * v0 + u[r][2] * v1 + u[r][3] * v2, E = u[r][4];
-                const double pe = (E - kin * (0.5 * gMs)) * gm1;
+                const double kin = fma(u[r][3], v2, fma(u[r][2], v1, u[r][1] * v0)), E = u[r][4];
+                const double eint = fma(kin, -0.5 * gMs, E);
                 u[r][0] = v0;
                 u[r][1] = v1;
                 u[r][2] = v2;
-                u[r][3] = (E + pe) * ir;
-                u[r][4] = v0 * v0 + v1 * v1 + v2 * v2;
+                u[r][3] = fma(eint, gm1, E) * ir;
+                u[r][4] = fma(v2, v2, fma(v1, v1, v0 * v0));
 #pragma unroll
                 for (int i = 0; i < 5; ++i) b[r][i] = 0.0;
             }
@@ -373,14 +376,14 @@ __device__ __forceinline__ void eul_volume(const EvalArgs& a, const double* tA, 
 #pragma unroll
                 for (int r = 0; r < NR; ++r) {
                     const double ud = u[r][DIR], h = u[r][3], usq = u[r][4];
-                    const double q = u[r][0] * g[r][1] + u[r][1] * g[r][2] + u[r][2] * g[r][3] + h * g[r][4];
-                    const double P = ud * g[r][4] + ph.ims * g[r][1 + DIR];
+                    const double q = fma(h, g[r][4], fma(u[r][2], g[r][3], fma(u[r][1], g[r][2], u[r][0] * g[r][1])));
+                    const double P = fma(ud, g[r][4], ph.ims * g[r][1 + DIR]);
                     const double kp = gMs * gm1 * P;
-                    b[r][0] += ud * q - 0.5 * kp * usq;
+                    b[r][0] = fma(ud, q, fma(-0.5 * kp, usq, b[r][0]));
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) b[r][1 + c] += kp * u[r][c] - ud * g[r][1 + c];
+                    for (int c = 0; c < 3; ++c) b[r][1 + c] = fma(kp, u[r][c], fma(-ud, g[r][1 + c], b[r][1 + c]));
                     b[r][1 + DIR] -= g[r][0] + q;
-                    b[r][4] -= gm1 * P + ud * g[r][4];
+                    b[r][4] = fma(-gm1, P, fma(-ud, g[r][4], b[r][4]));
                 }
             };
             dirn(std::integral_constant<int, 0>{});
@@ -413,22 +416,22 @@ __device__ __forceinline__ void eul_volume(const EvalArgs& a, const double* tA, 
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
                     w[r][c] = u[r][1 + c] * ir;
-                    kin += u[r][1 + c] * w[r][c];
+                    kin = fma(u[r][1 + c], w[r][c], kin);
                 }
-                const double pe = (u[r][4] - kin * (0.5 * gMs)) * gm1;
+                const double eint = fma(kin, -0.5 * gMs, u[r][4]);   // p / (gamma - 1)
                 if constexpr (MODE == MODE_JVP) {
                     double kt = 0.0;
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
-                        wt[r][c] = (vl[r][1 + c] - w[r][c] * vl[r][0]) * ir;
-                        kt += vl[r][1 + c] * w[r][c] + u[r][1 + c] * wt[r][c];
+                        wt[r][c] = fma(-w[r][c], vl[r][0], vl[r][1 + c]) * ir;
+                        kt = fma(vl[r][1 + c], w[r][c], fma(u[r][1 + c], wt[r][c], kt));
                     }
-                    const double pt = (vl[r][4] - kt * (0.5 * gMs)) * gm1;
-                    vl[r][0] = vl[r][4] + pt;
-                    vl[r][4] = pt * ph.ims;
+                    const double et = fma(kt, -0.5 * gMs, vl[r][4]);
+                    vl[r][0] = fma(et, gm1, vl[r][4]);
+                    vl[r][4] = et * gm1 * ph.ims;
                 }
-                u[r][0] = u[r][4] + pe;
-                u[r][4] = pe * ph.ims;
+                u[r][0] = fma(eint, gm1, u[r][4]);
+                u[r][4] = eint * gm1 * ph.ims;
             }
             auto dirn = [&](auto dc) {
                 constexpr int DIR = decltype(dc)::value;
@@ -442,15 +445,16 @@ __device__ __forceinline__ void eul_volume(const EvalArgs& a, const double* tA, 
                         if constexpr (MODE == MODE_RES) {
                             F[0] = u[r][1 + DIR];
 #pragma unroll
-                            for (int c = 0; c < 3; ++c) F[1 + c] = u[r][1 + c] * w[r][DIR];
-                            F[1 + DIR] += u[r][4];
+                            for (int c = 0; c < 3; ++c)
+                                F[1 + c] = c == DIR ? fma(u[r][1 + c], w[r][DIR], u[r][4]) : u[r][1 + c] * w[r][DIR];
                             F[4] = w[r][DIR] * u[r][0];
                         } else {
                             F[0] = vl[r][1 + DIR];
 #pragma unroll
-                            for (int c = 0; c < 3; ++c) F[1 + c] = vl[r][1 + c] * w[r][DIR] + u[r][1 + c] * wt[r][DIR];
-                            F[1 + DIR] += vl[r][4];
-                            F[4] = wt[r][DIR] * u[r][0] + w[r][DIR] * vl[r][0];
+                            for (int c = 0; c < 3; ++c)
+                                F[1 + c] = fma(vl[r][1 + c], w[r][DIR],
+                                               c == DIR ? fma(u[r][1 + c], wt[r][DIR], vl[r][4]) : u[r][1 + c] * wt[r][DIR]);
+                            F[4] = fma(wt[r][DIR], u[r][0], w[r][DIR] * vl[r][0]);
                         }
 #pragma unroll
                         for (int i = 0; i < 5; ++i) o[i * Q * SLV] = F[i] * f;

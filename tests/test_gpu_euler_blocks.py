@@ -131,3 +131,30 @@ def test_a_bad_density_reaches_the_cells_it_reaches_on_the_slab_kernel(speed, va
             sets.append([np.nonzero(~np.isfinite(t.cpu().numpy().reshape(J, -1)).all(axis=1))[0].tolist()
                          for t in (out, ev.jvp(u, v), ev.vjp(u, v))])
     assert sets[0] == sets[1]
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4])
+@pytest.mark.parametrize("n", [(10, 5, 4), (18, 17, 1), (9, 4, 3)], ids=lambda n: "x".join(map(str, n)))
+def test_euler_bits_do_not_depend_on_the_place_in_a_block(n, k):
+    """Ranges of planes cut the blocks differently; every cell keeps the bits of the whole-grid call, as
+    partitioned grids and the chunks of the host path rely on."""
+    import torch
+    op, g, dom, cod, U = make(n, k, C.CELLS_GENERATOR, 23, 0.1)
+    plane, npc = n[1] * n[2], 5 * dom[0].Np
+    u, v = torch.from_numpy(U).cuda(), torch.from_numpy(np.random.default_rng(3).uniform(-1, 1, U.size)).cuda()
+    st = ctypes.c_void_p(C.CUDA_STREAM_LEGACY)
+    with op.GetEvaluatorEx(dom, None, cod) as ev:
+        for mode in range(3):
+            args = (C.ptr(u), C.ptr(v) if mode else None)
+
+            def cells(lo, hi):
+                out = torch.zeros_like(u)
+                C.check(C.lib().bosss_b200_apply_device(ev.handle, mode, 1.0, 0.0, *args, C.ptr(out), 0.0, lo, hi, st))
+                torch.cuda.synchronize()
+                return out[lo * npc:hi * npc]
+
+            whole = cells(0, g.NoOfCells)
+            for size in (1, 2, 3, 5):
+                for p in range(0, n[0], size):
+                    lo, hi = p * plane, min(p + size, n[0]) * plane
+                    assert torch.equal(cells(lo, hi), whole[lo * npc:hi * npc]), (mode, size, p)
