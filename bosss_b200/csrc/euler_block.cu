@@ -55,6 +55,14 @@ ModalTile euler_tiling(const EvalArgs& a) {
 template <int K, int MODE>
 cudaError_t launch_euler(const EvalArgs& a, cudaStream_t s) {
     using C = EulerCfg<K, MODE>;
+    // J^T w for k = 2 on small grids: the slab tiles (4 cells, three CTAs per SM) take 15.6-20.7 us as long as they
+    // fit one wave, the blocks' chain of phases 16.6-21.3 us (us, slab / blocks: 8 cells 15.5 / 16.2, 512 cells
+    // 16.1 / 16.5, 729 cells 18.4 / 19.2, 1728 cells 20.7 / 21.3, 2744 cells 35.9 / 23.9); the other degrees and modes are
+    // faster in blocks at every size
+    if constexpr (K == 2 && MODE == MODE_VJP) {
+        static const KernelEntry* slab = registered(PHYS_EULER, 3, K, K + 1, MODE, VARIANT_SLAB);
+        if (slab && whole_grid_ctas(*slab, a.g) <= 148 * 3) return slab->launch(a, s);
+    }
     static unsigned long long done = 0ull;
     int dev = 0;
     cudaGetDevice(&dev);

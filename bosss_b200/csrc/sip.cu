@@ -59,9 +59,18 @@ template <int K, int Q, int MODE>
 cudaError_t launch_sip(const EvalArgs& a, cudaStream_t s) {
     using C = SipCfg<K, Q, MODE>;
     if (a.vol_flag || a.face_flag) {   // species masks: the slab tile reads them
-        auto it = kernel_registry().find(KernelKey(PHYS_SIP, 3, K, Q, MODE, VARIANT_SLAB));
-        if (it == kernel_registry().end()) return cudaErrorNotSupported;
-        return it->second.launch(a, s);
+        const KernelEntry* slab = registered(PHYS_SIP, 3, K, Q, MODE, VARIANT_SLAB);
+        return slab ? slab->launch(a, s) : cudaErrorNotSupported;
+    }
+    // Products with 7 or 9 nodes on the smallest grids: the generic tile spreads a cell's nodes over 128 or more
+    // threads, a block has a thread per z-slab and a chain of phases (24-28 us for k = 3, 41-57 us for k = 4
+    // whatever the size). As long as the generic tiles fit one wave -- one CTA per SM for k = 3, two for k = 4 --
+    // they are faster (us, generic / block; J v, J^T w within 1 us of it): k = 4, Q = 9, 8 cells 27.3 / 51.8, 216 cells
+    // 33.1 / 52.4, 343 cells (second wave) 56.7 / 48.5; Q = 7, 512 cells 38.2 / 41.1, 729 cells 66.1 / 43.8; k = 3, 1 cell
+    // 23.2 / 27.3, 216 cells 25.9 / 26.7, 343 cells 30.3 / 26.3
+    if constexpr (MODE != MODE_RES && Q >= 7) {
+        static const KernelEntry* generic = registered(PHYS_SIP, 3, K, Q, MODE, VARIANT_GENERIC);
+        if (generic && whole_grid_ctas(*generic, a.g) <= 148 * (K == 4 ? 2 : 1)) return generic->launch(a, s);
     }
     static const Tables1D V = [] {
         Tables1D t;

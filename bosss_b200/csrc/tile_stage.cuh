@@ -94,6 +94,19 @@ inline TileRange tile_range(const EvalArgs& a, int D) {
     return r;
 }
 
+// the quadrature kernel that a block kernel leaves some launches to; null: no instance
+inline const KernelEntry* registered(int phys, int D, int K, int Q, int mode, int variant) {
+    const auto it = kernel_registry().find(KernelKey(phys, D, K, Q, mode, variant));
+    return it == kernel_registry().end() ? nullptr : &it->second;
+}
+
+// CTAs of the kernel `e` over the whole grid (of a part: the global one, so that parts, cell ranges and the
+// whole grid take the same kernel)
+inline long long whole_grid_ctas(const KernelEntry& e, const GridConst& g) {
+    const long long J = (long long)g.gn[0] * g.gn[1] * g.gn[2];
+    return (J + e.cells_per_block - 1) / e.cells_per_block;
+}
+
 // memory-order view of a grid and the block of one tile
 struct TileGeom {
     bool rev;          // GlobalID order: x fastest

@@ -204,8 +204,9 @@ int bosss_b200_get_sizes(const bosss_handle* h, int64_t* n_domain_dofs, int64_t*
  * face terms (split-precision residual), 5 modal stencil kernel (scalar operators, linear with
  * constant coefficients, rule exact for them; automatic choice only), 6 face-once block kernel
  * of nonlinear SIP diffusion in 3D and 7 face-once block kernel
- * of the 3D Euler operator on periodic grids (both automatic choice only); and the kernel
- * launches of one whole-grid call. */
+ * of the 3D Euler operator on periodic grids (both automatic choice only; on their smallest
+ * grids some products of 6 and 7 run on the generic or slab kernel, as do evaluations with
+ * species masks); and the kernel launches of one whole-grid call. */
 int bosss_b200_kernel_info(const bosss_handle* h, int32_t mode, int32_t* kernel, int32_t* launches);
 
 /* EvaluatorNonLin.Evaluate (DifferentialOperator.cs:1584-1661):

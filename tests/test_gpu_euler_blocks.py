@@ -158,3 +158,19 @@ def test_euler_bits_do_not_depend_on_the_place_in_a_block(n, k):
                 for p in range(0, n[0], size):
                     lo, hi = p * plane, min(p + size, n[0]) * plane
                     assert torch.equal(cells(lo, hi), whole[lo * npc:hi * npc]), (mode, size, p)
+
+
+@pytest.mark.parametrize("n,slab", [((12, 37, 4), True), ((1777, 1, 1), False)], ids=["1776_cells", "1777_cells"])
+def test_small_grid_rule_of_the_quadratic_adjoint(n, slab):
+    """J^T w for k = 2 runs on the slab tiles as long as these fit one wave (1776 cells): its bits below
+    the line, blocks that match the oracle from there on."""
+    import torch
+    op, g, dom, cod, U = make(n, 2, C.CELLS_GENERATOR, 9, 0.5)
+    W = np.random.default_rng(2).uniform(-1, 1, U.size)
+    u, w = torch.from_numpy(U).cuda(), torch.from_numpy(W).cuda()
+    got = []
+    for kernel in (C.KERNEL_AUTO, C.KERNEL_SLAB):
+        with op.GetEvaluatorEx(dom, None, cod, kernel=kernel) as ev:
+            got.append(ev.vjp(u, w))
+    assert torch.equal(*got) == slab
+    assert rel(got[0].cpu().numpy(), orc.vjp(op.descriptor([2] * 5, [2] * 5, 3), g.desc(), U, W)) <= TOL

@@ -83,3 +83,24 @@ def test_sip_blocks_cell_ranges():
                 want = torch.full_like(U, 9.0)
                 want[lo * Np:hi * Np] = whole[lo * Np:hi * Np]
                 assert torch.equal(c, want), (mode, lo, hi)
+
+
+@pytest.mark.parametrize("k,q,small,large", [(3, 7, (8, 37, 1), (11, 27, 1)), (4, 7, (16, 37, 1), (1, 593, 1)),
+                                             (4, 9, (8, 37, 1), (11, 27, 1))])
+def test_products_on_both_sides_of_the_small_grid_rule(k, q, small, large):
+    """J v and J^T w with 7 or 9 nodes run on the generic tiles as long as these fit one wave (296 or 592
+    cells): its bits below the line, blocks that match the oracle from there on."""
+    import torch
+    for n in (small, large):
+        op, g, dom, cod = make(n, k, q, (True, False, True), 1)
+        desc = (op.descriptor([k], [k], 3), g.desc())
+        r = np.random.default_rng(k)
+        U, V = (r.uniform(-1, 1, g.NoOfCells * dom[0].Np) for _ in range(2))
+        u, v = torch.from_numpy(U).cuda(), torch.from_numpy(V).cuda()
+        got = []
+        for kernel in (C.KERNEL_AUTO, C.KERNEL_GENERIC):
+            with op.GetEvaluatorEx(dom, None, cod, kernel=kernel) as ev:
+                got.append([ev.jvp(u, v), ev.vjp(u, v)])
+        assert all(torch.equal(a, b) for a, b in zip(*got)) == (n == small)
+        for t, f in zip(got[0], (orc.jvp, orc.vjp)):
+            assert rel(t.cpu().numpy(), f(*desc, U, V)) <= TOL
