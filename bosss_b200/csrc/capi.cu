@@ -838,8 +838,9 @@ static int host_pipelined(bosss_handle* h, const HostJob* jobs, int njobs, const
     for (int k = 0; k < njobs; ++k)   // split-precision residuals evaluate the whole grid at once
         if (jobs[k].mode == MODE_RES && h->precision == BOSSS_PRECISION_SPLIT_FP32) nch = 1;
     if (nch < 1) nch = 1;
-    // two streams only for kernels without scratch of the handle (face-once buffer, tensor-core path)
-    const bool two = njobs > 1 && !h->faces_once && h->precision == BOSSS_PRECISION_FP64;
+    // two streams only for kernels without scratch of the handle (face-once buffer, tensor-core path), and for
+    // several chunks: a small call gains nothing and pays the second set of events (Euler 2^3 k=1 3 us of 80)
+    const bool two = njobs > 1 && nch > 1 && !h->faces_once && h->precision == BOSSS_PRECISION_FP64;
     if (!h->s_in) CUDA_TRY(cudaStreamCreateWithFlags(&h->s_in, cudaStreamNonBlocking));
     if (!h->s_out) CUDA_TRY(cudaStreamCreateWithFlags(&h->s_out, cudaStreamNonBlocking));
     for (int c = 0; c < nch; ++c) {
@@ -889,8 +890,7 @@ static int host_pipelined(bosss_handle* h, const HostJob* jobs, int njobs, const
     for (int c = 0; c < nch; ++c) {
         for (int k = 0; k < njobs; ++k) {
             cudaStream_t sk = k > 0 && two ? h->s_second : s;
-            cudaEvent_t done = k > 0 && two ? h->ev_second[c] : h->ev_done[c];
-            e = cudaStreamWaitEvent(sk, h->ev_in[c], 0);
+            if (k == 0 || two) e = cudaStreamWaitEvent(sk, h->ev_in[c], 0);
             if (e != cudaSuccess) return finish(fail(BOSSS_ERR_CUDA, cudaGetErrorString(e)));
             EvalArgs a = h->base;
             a.U = h->dU;
@@ -903,12 +903,16 @@ static int host_pipelined(bosss_handle* h, const HostJob* jobs, int njobs, const
             a.cend = first_plane(c + 1) * pc;
             rc = launch_eval(h, jobs[k].mode, a, sk);
             if (rc) return finish(rc);
+            if (!two && k + 1 < njobs) continue;   // one stream: the outputs leave together
+            cudaEvent_t done = k > 0 && two ? h->ev_second[c] : h->ev_done[c];
             e = cudaEventRecord(done, sk);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(so, done, 0);
-            const long long c0 = first_plane(c) * pc, n = (first_plane(c + 1) - first_plane(c)) * pc, m = nY(jobs[k]);
-            if (e == cudaSuccess)
-                e = cudaMemcpyAsync(jobs[k].Y + c0 * m, jobs[k].dY + c0 * m, sizeof(double) * n * m, cudaMemcpyDeviceToHost,
+            const long long c0 = first_plane(c) * pc, n = (first_plane(c + 1) - first_plane(c)) * pc;
+            for (int q = two ? k : 0; q <= k && e == cudaSuccess; ++q) {
+                const long long m = nY(jobs[q]);
+                e = cudaMemcpyAsync(jobs[q].Y + c0 * m, jobs[q].dY + c0 * m, sizeof(double) * n * m, cudaMemcpyDeviceToHost,
                                     so);
+            }
             if (e != cudaSuccess) return finish(fail(BOSSS_ERR_CUDA, cudaGetErrorString(e)));
         }
     }
